@@ -102,6 +102,11 @@ void push_layer_learn(const bm_area_s* A, uint32_t i, std::vector<Step>& out) {
     }
 }
 
+// Tuft t of data layer i may fold into its layer's tail, a thread per cell.
+bool cell_tuft(const bm_area_s* A, uint32_t i, uint32_t t) {
+    return !A->fused.t[i][t].ok && A->plan.layers[i].tufts[t].syns_per_tft <= kCellTuftSyns;
+}
+
 // Slices of data layer i are plain: unscaled, unshifted and laid out back to
 // back from the layer's first axon, so the axon a control writes for cell c
 // is axn_idz + c.
@@ -125,12 +130,12 @@ void fuse_steps(const bm_area_s* A, std::vector<Step>& v, bool fold_cell_tufts) 
     std::vector<Step> out;
     for (size_t k = 0; k < v.size(); k++) {
         const Step& s = v[k];
-        // A spiny stellate tuft whose cells have one dendrite, taken by the
-        // fused kernel, also runs the ssc_cycle that follows it (arg 1): the
-        // soma is that dendrite's state, known in the same launch.
+        // A spiny stellate tuft whose cells have one dendrite also runs the
+        // ssc_cycle that follows it (arg 1): the soma is that dendrite's
+        // state, known in the same launch.
         if (s.kind == ST_TUFT && k + 1 < v.size() && v[k + 1].kind == ST_SSC_CYCLE && v[k + 1].layer == s.layer &&
             P.layers[s.layer].kind == BM_LYR_SPINY_STELLATE && P.layers[s.layer].n_tufts == 1 &&
-            P.layers[s.layer].tufts[0].dens_per_tft == 1 && A->fused.t[s.layer][s.idx].ok) {
+            P.layers[s.layer].tufts[0].dens_per_tft == 1) {
             out.push_back({ST_TUFT, s.layer, s.idx, 1});
             k++;
             continue;
@@ -162,8 +167,8 @@ void fuse_steps(const bm_area_s* A, std::vector<Step>& v, bool fold_cell_tufts) 
             }
             const bool learn = n_dst > 0 && all;
             if (learn || m == j) {
-                // The layer's tuft steps that run per cell (tufts the fused
-                // kernel does not take) come right before its soma step with
+                // The layer's tuft steps of a few synapses a cell (see
+                // cell_tuft) come right before its soma step with
                 // only other tuft steps of the layer in between, which write
                 // no axon: they fold into the tail, each cell's four stages
                 // ahead of its soma.
@@ -171,7 +176,7 @@ void fuse_steps(const bm_area_s* A, std::vector<Step>& v, bool fold_cell_tufts) 
                 for (size_t q = out.size(); q > 0 && fold_cell_tufts; q--) {
                     const Step& o = out[q - 1];
                     if (o.kind != ST_TUFT || o.layer != s.layer) break;
-                    if (!A->fused.t[s.layer][o.idx].ok && o.idx < 8) tufts |= (uint8_t)(1u << o.idx);
+                    if (cell_tuft(A, s.layer, o.idx) && o.idx < 8) tufts |= (uint8_t)(1u << o.idx);
                 }
                 if (tufts)
                     out.erase(std::remove_if(out.begin(), out.end(),
@@ -203,9 +208,9 @@ uint64_t bm::cell_tuft_cells(const bm_area_s* A) {
     uint64_t n = 0;
     for (uint32_t i = 0; i < P.n_layers; i++) {
         if (P.layers[i].kind != BM_LYR_PYRAMIDAL) continue;
-        bool cell_tuft = false;
-        for (uint32_t t = 0; t < P.layers[i].n_tufts; t++) cell_tuft |= !A->fused.t[i][t].ok;
-        if (cell_tuft) n += P.layers[i].cells;
+        bool any = false;
+        for (uint32_t t = 0; t < P.layers[i].n_tufts; t++) any |= cell_tuft(A, i, t);
+        if (any) n += P.layers[i].cells;
     }
     return n;
 }
@@ -259,7 +264,9 @@ void bm::exec_step(bm_area_s* A, const Step& st, cudaStream_t s, bool end_cycle)
             run(K_FUSED_TUFT,
                 [&] { launch_fused_tuft(A->fused, A->axns(), A->slices, D, i, x, A->ctl, s, (st.arg & 1) != 0, host_cycle); });
         } else {
-            run(K_TUFT_CELLS, [&] { launch_tuft_cells(A->axns(), A->slices, D, x, A->ctl, s); });
+            run(K_TUFT_SEG, [&] {
+                launch_tuft_seg(A->axns(), A->slices, D, x, A->ctl, A->fused.sms, (st.arg & 1) != 0, s, host_cycle);
+            });
         }
         break;
     case ST_INHIB_MTP:
@@ -465,14 +472,13 @@ void bm::note_sources(bm_area_s* A, uint32_t i, uint64_t b, uint64_t e, const ui
 
 namespace {
 
-// A step the front stream can take: a spatial layer's fused tuft (with its
-// folded soma step) or its inhibition with learning; their kernels take the
-// cycle number from the host.
+// A step the front stream can take: a spatial layer's tuft (with its folded
+// soma step) or its inhibition with learning; their kernels take the cycle
+// number from the host.
 bool front_step_ok(const bm_area_s* A, const Step& st) {
     const bm_area_plan& P = A->plan;
     if (!(P.layers[st.layer].tags & BM_TAG_SPATIAL)) return false;
-    if (st.kind == ST_TUFT) return A->fused.t[st.layer][st.idx].ok;
-    return st.kind == ST_INHIB_MTP;
+    return st.kind == ST_TUFT || st.kind == ST_INHIB_MTP;
 }
 
 // What a frame intake writes: the axon slices of every input.
@@ -779,6 +785,7 @@ void bm::fill_dev_layer(DevLayer& D, const bm_area_plan& P, uint32_t i, uint8_t*
     D.dst_id = L.bsl_dst_tft_id;
     D.apc_id = L.apc_dst_tft_id;
     D.n_syns = L.n_syns;
+    D.n_slices = P.n_slices;
     for (int k = 0; k < BM_BUF_COUNT; k++)
         D.buf[k] = L.buf_off[k] == UINT64_MAX ? nullptr : slab + L.buf_off[k];
     for (uint32_t t = 0; t < L.n_tufts; t++) {
@@ -790,6 +797,7 @@ void bm::fill_dev_layer(DevLayer& D, const bm_area_plan& P, uint32_t i, uint8_t*
         DT.mad_l2 = T.max_active_dens_l2;
         DT.thresh = T.den_threshold;
         DT.den_kind = T.den_kind;
+        DT.src_slc = T.n_src_uniq ? T.src_uniq_slc_ids[0] : 0;
         DT.syn_idz = T.syn_idz;
         DT.den_idz = T.den_idz;
         DT.cel_idz = T.cel_idz;

@@ -18,12 +18,12 @@ namespace bm {
 enum Kind {
     K_SYN_FLAGS, K_SYN_CYCLE, K_DEN_CYCLE, K_TFT_CYCLE, K_SSC_CYCLE, K_INHIB_SIMPLE, K_INHIB_PASS,
     K_SSC_MTP, K_PYR_CYCLE, K_PYR_OUTPUT, K_INTRA_COL, K_TFT_DST_MTP, K_CYCLE_END, K_INTAKE,
-    K_FUSED_TUFT, K_TUFT_CELLS, K_INHIB_MTP, K_PYR_TAIL, K_REGROW, K_SMOOTH, K_RETINA, K_COUNT
+    K_FUSED_TUFT, K_TUFT_SEG, K_INHIB_MTP, K_PYR_TAIL, K_REGROW, K_SMOOTH, K_RETINA, K_COUNT
 };
 const char* const kKindNames[K_COUNT] = {
     "tft_set_syn_flags", "syn_cycle", "den_cycle_tft", "tft_cycle", "ssc_cycle", "inhib_simple",
     "inhib_passthrough", "ssc_mtp_simple", "pyr_cycle", "pyr_output", "inhib_intra_column", "tft_dst_mtp",
-    "cycle_end", "intake", "fused_tuft_cycle", "tuft_cells", "inhib_mtp", "pyr_tail", "regrow",
+    "cycle_end", "intake", "fused_tuft_cycle", "tuft_seg", "inhib_mtp", "pyr_tail", "regrow",
     "smooth_activity", "retina"};
 
 struct DevGuard {
@@ -292,8 +292,10 @@ namespace bm {
 // tail (one launch fewer; worth it while that work is small, see
 // kFoldCellTufts), else they stay steps of their own.
 void area_steps(const bm_area_s* A, std::vector<Step>& out, bool fold_cell_tufts);
-// Cells of the pyramidal layers with per-cell (unfused) tufts: up to this many
-// (over an area, or over a batch's areas) those tufts fold into the tail.
+// Tufts of at most kCellTuftSyns synapses a cell that the fused kernel does
+// not take may run inside their layer's tail: while the layers' cells that
+// have them number up to kFoldCellTufts (over an area, or over a batch's
+// areas) they do.
 // Beyond it they stay a step of their own, which overlaps a side-stream tuft
 // step where the tail, after the streams join, would not.
 constexpr uint64_t kFoldCellTufts = 16384;

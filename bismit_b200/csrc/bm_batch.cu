@@ -33,6 +33,7 @@
 
 #include "bm_area.h"
 #include "bm_items.cuh"
+#include "bm_seg.cuh"
 
 using namespace bm;
 
@@ -49,6 +50,7 @@ struct CellJob {
     int32_t ctrl;       // pyramidal tail: 0 none, 1 intra-column, 2 output
     uint32_t learn;     // fused steps: learning included
     uint32_t x;         // tuft or control index
+    uint32_t per;       // BK_TUFT_SEG: cells a block
     uint32_t tufts;     // pyramidal tail: per-cell tufts folded in (bit t)
     uint32_t n;         // work items (cells or columns)
     uint32_t block0;    // first block of this job
@@ -70,8 +72,9 @@ struct BatchCtl {
     uint64_t frame_bytes;    // bytes of one cycle's block
 };
 
-// An unfused tuft's four stages, one thread per cell (tuft_cell_item).
-constexpr int BK_TUFT_CELLS = 100;
+// An unfused tuft's stages: by 16- or 4-byte windows (bm_seg.cuh), or a thread
+// per cell (tuft_cell_item; tufts of a few synapses).
+constexpr int BK_TUFT_SEG16 = 100, BK_TUFT_SEG4 = 101, BK_TUFT_CELLS = 102;
 
 constexpr uint32_t kCellBlock = 128;
 constexpr uint32_t kIntakeBlock = 256;
@@ -124,6 +127,16 @@ __global__ void __launch_bounds__(kCellBlock)
         break;
     default: break;
     }
+}
+
+template <int W>
+__global__ void __launch_bounds__(kSegBlock) k_batch_tuft_seg(const CellJob* __restrict__ jobs, uint32_t n_jobs) {
+    pdl_begin();
+    __shared__ SegSmem S;
+    const CellJob& J = jobs[block_job(jobs, n_jobs)];
+    const uint32_t c0 = (blockIdx.x - J.block0) * J.per;
+    tuft_seg_block<W>(J.axns, J.slices, J.L, J.x, rnd_at(J.L.tft[J.x].rnd_key_den, J.ctl->cycle), c0,
+                      min(J.per, J.n - c0), (J.learn & 1) != 0, S);
 }
 
 __global__ void __launch_bounds__(kIntakeBlock)
@@ -182,6 +195,8 @@ void launch_cells(int st, const CellJob* jobs, uint32_t n_jobs, uint32_t n_block
         BM_CELLS(ST_INHIB_MTP)
     case ST_PYR_TAIL: launch_pdl(k_batch_tail, n_blocks, kCellBlock, 0, s, jobs, n_jobs); break;
         BM_CELLS(BK_TUFT_CELLS)
+    case BK_TUFT_SEG16: launch_pdl(k_batch_tuft_seg<16>, n_blocks, kSegBlock, 0, s, jobs, n_jobs); break;
+    case BK_TUFT_SEG4: launch_pdl(k_batch_tuft_seg<4>, n_blocks, kSegBlock, 0, s, jobs, n_jobs); break;
 #undef BM_CELLS
     default: break;
     }
@@ -376,7 +391,9 @@ int add_cells(bm_ctx ctx, bm_batch_s::StepPlan& p, int k) {
         if (n > 0xFFFFFFFFull) return set_err(BM_ERR_UNSUPPORTED, "batched step of more than 2^32 items");
         J.n = (uint32_t)n;
         J.block0 = (uint32_t)blocks;
-        blocks += (n + kCellBlock - 1) / kCellBlock;
+        J.per = kCellBlock;
+        if (k == BK_TUFT_SEG16 || k == BK_TUFT_SEG4) J.per = seg_cells(J.L.tft[st.idx].spt, k == BK_TUFT_SEG16 ? 16 : 4);
+        blocks += (n + J.per - 1) / J.per;
         jobs.push_back(J);
     }
     if (blocks > 0x7FFFFFFFull) return set_err(BM_ERR_UNSUPPORTED, "batched step of too many blocks");
@@ -477,9 +494,17 @@ int build_step(bm_ctx ctx, bm_batch_s::StepPlan& p) {
         return build_fused(p);
     }
     if (!none_ok) return BM_OK;
-    // No area can take the fused kernel here (e.g. one-synapse dendrites):
-    // the tuft's four stages per cell, batched.
-    return add_cells(ctx, p, BK_TUFT_CELLS);
+    // No area can take the fused kernel here (e.g. one-synapse dendrites).
+    uint64_t n = 0;
+    int sms = 148;
+    bool tiny = (st.arg & 1) == 0;
+    for (auto& [A, t] : p.tufts) {
+        tiny = tiny && A->plan.layers[st.layer].tufts[t].syns_per_tft <= kCellTuftSyns;
+        n += (uint64_t)A->plan.layers[st.layer].cells * A->plan.layers[st.layer].tufts[t].syns_per_tft;
+        sms = A->fused.sms;
+    }
+    if (tiny) return add_cells(ctx, p, BK_TUFT_CELLS);
+    return add_cells(ctx, p, seg_window(n, sms) == 16 ? BK_TUFT_SEG16 : BK_TUFT_SEG4);
 }
 
 // Consecutive batched tuft steps of one layer touch disjoint buffers: one

@@ -59,6 +59,7 @@ typedef uint4 SliceRec;
 
 struct DevTuft {
     uint32_t dpt, spd, spt, mad_l2, thresh, den_kind;
+    uint32_t src_slc;       // first source slice of the tuft's pool
     uint64_t syn_idz, den_idz, cel_idz;
     uint64_t rnd_key_den;   // den_cycle_tft per-launch value key
     uint64_t rnd_key_mtp;   // tft_dst_mtp per-launch value key
@@ -66,6 +67,7 @@ struct DevTuft {
 
 struct DevLayer {
     uint32_t kind, depth, v_size, u_size, cells, base_slc, axn_idz, n_tufts;
+    uint32_t n_slices;      // of the area's slice table
     uint32_t enabled_flags, prx_id, dst_id, apc_id;
     uint64_t n_syns;
     uint8_t* buf[BM_BUF_COUNT];
@@ -146,6 +148,29 @@ __device__ __forceinline__ uint8_t update_activity(uint8_t act, int is_active, i
 // syn_fire, cl/syns.cl:2-4.
 __device__ __forceinline__ uint8_t syn_fire(uint8_t a) {
     return (uint8_t)(((a != 0) << 7) + (a >> kSynapseAxonBiasLog2));
+}
+
+// 0xFF in every byte of x whose sign bit is set (prmt's sign-replicate mode).
+__device__ __forceinline__ uint32_t neg_bytes(uint32_t x) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, 0xBA98;" : "=r"(r) : "r"(x), "r"(0u));
+    return r;
+}
+// 0x80 in every byte of x that is non-zero.
+__device__ __forceinline__ uint32_t nz_bytes(uint32_t x) {
+    return (((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u;
+}
+
+// ssc_cycle (cl/bismit.cl:849-884) folded into the spiny stellate tuft stage
+// for cells of one dendrite, whose soma state is that dendrite's state: from
+// cell c's energy and the dendrite state just computed, writes the energy and
+// returns the soma state.
+__device__ __forceinline__ uint32_t ssc_soma(uint8_t* en, uint32_t c, uint32_t energy, uint32_t state) {
+    const int active = state != 0;
+    const int restless = (energy > 191) & active;
+    const int dark = energy == 255;
+    en[c] = (uint8_t)((dark | restless) ? energy - 64 : energy);
+    return min(state + (uint32_t)restless * 255u + (uint32_t)dark * 255u, 255u);
 }
 
 // axn_idx_3d_unsafe (cl/bismit.cl:323-363, scalar: the slice mid is added to

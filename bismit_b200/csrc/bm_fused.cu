@@ -243,33 +243,10 @@ __device__ __forceinline__ bool consumers_sync_or(bool p) {
 }
 
 // ------------------------------------------------------------ helpers ----
-// 0xFF in every byte of x whose sign bit is set (prmt's sign-replicate mode).
-__device__ __forceinline__ uint32_t sign_bytes(uint32_t x) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, %2, 0xBA98;" : "=r"(r) : "r"(x), "r"(0u));
-    return r;
-}
 // The low bytes of a0..a3 as one word (a0 lowest).
 __device__ __forceinline__ uint32_t pack4(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
     return __byte_perm(__byte_perm(a0, a1, 0x0040), __byte_perm(a2, a3, 0x0040), 0x5410);
 }
-__device__ __forceinline__ uint32_t nz_bits(uint32_t x) {
-    // 0x80 in every byte of x that is non-zero.
-    return (((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u;
-}
-
-// ssc_cycle (cl/bismit.cl:849-884) folded into the spiny stellate tuft stage
-// for cells of one dendrite, whose soma state is that dendrite's state: from
-// cell c's energy and the dendrite state just computed, writes the energy and
-// returns the soma state.
-__device__ __forceinline__ uint32_t ssc_soma(uint8_t* en, uint32_t c, uint32_t energy, uint32_t state) {
-    const int active = state != 0;
-    const int restless = (energy > 191) & active;
-    const int dark = energy == 255;
-    en[c] = (uint8_t)((dark | restless) ? energy - 64 : energy);
-    return min(state + (uint32_t)restless * 255u + (uint32_t)dark * 255u, 255u);
-}
-
 __device__ __forceinline__ uint8_t gather_general(const FusedTuftArgs& A, uint32_t slc, uint32_t v, uint32_t u,
                                                   int vo, int uo) {
     bool safe;
@@ -319,9 +296,9 @@ __device__ __forceinline__ void finish_chunk(const FusedTuftArgs& A, const uint4
 #pragma unroll
         for (int w = 0; w < 4; w++) {
             const uint32_t keep = flags_clean ? 0u : (flw[w] & 0xEFEFEFEFu);
-            nflw[w] = keep | (nz_bits(stw[w]) >> 3);
+            nflw[w] = keep | (nz_bytes(stw[w]) >> 3);
             raw = __dp4a(nstw[w], 0x01010101u, raw);
-            sum = __dp4a(nstw[w] & ~sign_bytes(strw[w]), 0x01010101u, sum);
+            sum = __dp4a(nstw[w] & ~neg_bytes(strw[w]), 0x01010101u, sum);
         }
         *(uint4*)(A.st + off) = nst4;
         *(uint4*)(A.fl + off) = nfl4;
@@ -529,7 +506,7 @@ __device__ __forceinline__ int32_t footprint_base(const FusedTuftArgs& A, const 
 }
 
 // syn_fire of four packed axon bytes (cl/syns.cl:2-4).
-__device__ __forceinline__ uint32_t fire4(uint32_t x) { return nz_bits(x) | ((x >> 1) & 0x7F7F7F7Fu); }
+__device__ __forceinline__ uint32_t fire4(uint32_t x) { return nz_bytes(x) | ((x >> 1) & 0x7F7F7F7Fu); }
 
 // A footprint the tensor load brought in holds raw axon bytes: fire them in
 // place (consumer threads, 16 bytes each per step; the box is a multiple of
@@ -782,9 +759,9 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
             }
 #pragma unroll
             for (int w = 0; w < 4; w++) {
-                nfl[w] = nz_bits(stw[w]) >> 3;
+                nfl[w] = nz_bytes(stw[w]) >> 3;
                 raw = __dp4a(nst[w], 0x01010101u, raw);
-                sum = __dp4a(nst[w] & ~sign_bytes(strw[w]), 0x01010101u, sum);
+                sum = __dp4a(nst[w] & ~neg_bytes(strw[w]), 0x01010101u, sum);
             }
             *(uint4*)(A.st + off) = make_uint4(nst[0], nst[1], nst[2], nst[3]);
             *(uint4*)(A.fl + off) = make_uint4(nfl[0], nfl[1], nfl[2], nfl[3]);

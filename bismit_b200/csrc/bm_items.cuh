@@ -48,15 +48,13 @@ __device__ __forceinline__ void den_cycle_item(const DevLayer& L, uint32_t t, in
     L.buf[BM_BUF_DEN_STATES][di] = (uint8_t)min(sum >> 4, 255);
 }
 
-// tft_cycle, cl/bismit.cl:755-842; cell c of tuft t.
-__device__ __forceinline__ void tft_cycle_item(const DevLayer& L, uint32_t t, uint32_t c) {
-    const DevTuft& T = L.tft[t];
-    const uint8_t* sraw = L.buf[BM_BUF_DEN_STATES_RAW];
-    const uint8_t* sden = L.buf[BM_BUF_DEN_STATES];
-    uint64_t d0 = T.den_idz + (uint64_t)c * T.dpt;
+// tft_cycle, cl/bismit.cl:755-842; cell c of tuft T, whose dendrites' raw
+// states and states are at sraw and sden.
+__device__ __forceinline__ void tft_cycle_of(const DevLayer& L, const DevTuft& T, uint32_t c, const uint8_t* sraw,
+                                             const uint8_t* sden) {
     uint32_t best_id = 0, best_raw = 0, best_st = 0, sum = 0;
     for (uint32_t d = 0; d < T.dpt; d++) {
-        uint32_t r = sraw[d0 + d], s = sden[d0 + d];
+        uint32_t r = sraw[d], s = sden[d];
         if (r > best_raw) { best_id = d; best_raw = r; }
         best_st = max(best_st, s);
         sum += s;
@@ -72,6 +70,11 @@ __device__ __forceinline__ void tft_cycle_item(const DevLayer& L, uint32_t t, ui
     L.buf[BM_BUF_TFT_BEST_DEN_STATES_RAW][ci] = (uint8_t)best_raw;
     L.buf[BM_BUF_TFT_BEST_DEN_STATES][ci] = (uint8_t)best_st;
     L.buf[BM_BUF_TFT_STATES][ci] = state;
+}
+__device__ __forceinline__ void tft_cycle_item(const DevLayer& L, uint32_t t, uint32_t c) {
+    const DevTuft& T = L.tft[t];
+    const uint64_t d0 = T.den_idz + (uint64_t)c * T.dpt;
+    tft_cycle_of(L, T, c, L.buf[BM_BUF_DEN_STATES_RAW] + d0, L.buf[BM_BUF_DEN_STATES] + d0);
 }
 
 // ssc_cycle, cl/bismit.cl:849-884 (soma = the dendrite state buffer).

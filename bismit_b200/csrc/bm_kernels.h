@@ -132,15 +132,19 @@ void launch_smooth(const DevLayer& L, const int32_t* centers, uint32_t n, int32_
 // input grid to slices base_slc.. of `out`, each at its slice-table offset.
 void launch_retina(const uint8_t* in, uint8_t* out, const SliceRec* slices, uint32_t base_slc, uint32_t depth,
                    uint32_t v_size, uint32_t u_size, cudaStream_t s);
-// Fused cell steps (bm_items.cuh): an unfused tuft's four stages per cell;
-// inhibition with spiny stellate learning; pyramidal soma, control and distal
-// learning per column (ctrl: 0 none, 1 intra-column, 2 output).
-void launch_tuft_cells(const uint8_t* axns, const SliceRec* slices, const DevLayer& L, uint32_t t,
-                       const AreaCtl* ctl, cudaStream_t s);
+// Tufts of up to this many synapses a cell run a thread per cell
+// (tuft_cell_item) where the fused kernel does not take them.
+constexpr uint32_t kCellTuftSyns = 4;
+// A tuft the fused kernel does not take, every stage in one launch
+// (bm_seg.cuh), with ssc_cycle where `soma`.
+void launch_tuft_seg(const uint8_t* axns, const SliceRec* slices, const DevLayer& L, uint32_t t, const AreaCtl* ctl,
+                     int sms, bool soma, cudaStream_t s, int64_t host_cycle = -1);
+// Fused cell steps (bm_items.cuh): inhibition with spiny stellate learning;
+// pyramidal soma, control and distal learning per column (ctrl: 0 none, 1
+// intra-column, 2 output).
 void launch_inhib_mtp(uint8_t* axns, const SliceRec* slices, const DevLayer& L, int radius, uint64_t key,
                       bool learn, const AreaCtl* ctl, cudaStream_t s, int64_t host_cycle = -1);
-// `tufts` (bit t): tufts the fused tuft kernel does not take, run per cell
-// first; `end`: the last block to finish also ends the cycle.
+// `tufts` (bit t): tufts of a few synapses run per cell first; `end`: the last block to finish also ends the cycle.
 void launch_pyr_tail(uint8_t* axns, const SliceRec* slices, const DevLayer& L, int ctrl, bool learn, AreaCtl* ctl,
                      cudaStream_t s, uint32_t tufts = 0, bool end = false);
 void launch_tft_dst_mtp_plain(const uint8_t* axns, const DevLayer& L, uint32_t t, const AreaCtl* ctl,

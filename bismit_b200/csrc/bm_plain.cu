@@ -4,6 +4,7 @@
 // kernels (bm_fused.cu) must produce identical bytes.
 #include "bm_items.cuh"
 #include "bm_kernels.h"
+#include "bm_seg.cuh"
 
 namespace bm {
 
@@ -105,11 +106,28 @@ __global__ void k_tft_dst_mtp(const uint8_t* __restrict__ axns, DevLayer L, uint
     if (c < L.cells) tft_dst_mtp_item(axns, L, t, rnd_at(L.tft[t].rnd_key_mtp, ctl->cycle), c);
 }
 
+// Tufts of at most kCellTuftSyns synapses a cell, a thread per cell: 28,800
+// one-synapse cells take 7.9 us cold, in k_tuft_seg's blocks 15.6 us (57 of
+// them, each walking four cells a thread through its three steps).
 __global__ void k_tuft_cells(const uint8_t* __restrict__ axns, const SliceRec* __restrict__ slices, DevLayer L,
                              uint32_t t, const AreaCtl* ctl) {
     pdl_begin();
     uint32_t c = (uint32_t)gtid();
     if (c < L.cells) tuft_cell_item(axns, slices, L, t, rnd_at(L.tft[t].rnd_key_den, ctl->cycle), c);
+}
+
+// W: bytes of each thread's window (bm_seg.cuh). 16 while that still gives
+// every SM several blocks, else 4.
+template <int W>
+__global__ void __launch_bounds__(kSegBlock) k_tuft_seg(const uint8_t* __restrict__ axns,
+                                                        const SliceRec* __restrict__ slices, DevLayer L, uint32_t t,
+                                                        const AreaCtl* ctl, uint32_t per, int soma,
+                                                        long long host_cycle) {
+    pdl_begin();
+    __shared__ SegSmem S;
+    const uint32_t c0 = blockIdx.x * per;
+    const unsigned long long cyc = host_cycle >= 0 ? (unsigned long long)host_cycle : ctl->cycle;
+    tuft_seg_block<W>(axns, slices, L, t, rnd_at(L.tft[t].rnd_key_den, cyc), c0, min(per, L.cells - c0), soma != 0, S);
 }
 
 // Warp-cooperative: no thread leaves before the warp's shared part. With
@@ -295,9 +313,15 @@ void launch_retina(const uint8_t* in, uint8_t* out, const SliceRec* slices, uint
 void launch_inhib_intra_column_plain(uint8_t* axns, const SliceRec* slices, const DevLayer& L, cudaStream_t s) {
     launch_pdl(k_inhib_intra_column, nblk((uint64_t)L.v_size * L.u_size, 256), 256, 0, s, axns, slices, L);
 }
-void launch_tuft_cells(const uint8_t* axns, const SliceRec* slices, const DevLayer& L, uint32_t t,
-                       const AreaCtl* ctl, cudaStream_t s) {
-    launch_pdl(k_tuft_cells, nblk(L.cells, 128), 128, 0, s, axns, slices, L, t, ctl);
+void launch_tuft_seg(const uint8_t* axns, const SliceRec* slices, const DevLayer& L, uint32_t t, const AreaCtl* ctl,
+                     int sms, bool soma, cudaStream_t s, int64_t host_cycle) {
+    if (L.tft[t].spt <= kCellTuftSyns && !soma && host_cycle < 0) {
+        launch_pdl(k_tuft_cells, nblk(L.cells, 128), 128, 0, s, axns, slices, L, t, ctl);
+        return;
+    }
+    const uint32_t W = seg_window((uint64_t)L.cells * L.tft[t].spt, sms), per = seg_cells(L.tft[t].spt, W);
+    launch_pdl(W == 16 ? k_tuft_seg<16> : k_tuft_seg<4>, nblk(L.cells, per), kSegBlock, 0, s, axns, slices, L, t, ctl,
+               per, soma ? 1 : 0, (long long)host_cycle);
 }
 void launch_inhib_mtp(uint8_t* axns, const SliceRec* slices, const DevLayer& L, int radius, uint64_t key,
                       bool learn, const AreaCtl* ctl, cudaStream_t s, int64_t host_cycle) {

@@ -1,0 +1,75 @@
+"""The tuft kernel for shapes the tiled one does not take (bm_seg.cuh), against
+the oracle on the whole slab (tolerance: exact): synapse ranges off 16-byte
+alignment, dendrites and cells of odd lengths, cells larger than a block's
+piece, scaled and nonspatial sources, both window widths, and the batched
+form."""
+import numpy as np
+import pytest
+
+import oracle
+from bismit_b200 import configs, cortex, map as M
+from helpers import diff_report, frames_for, initial_slab, settings_for
+
+pytestmark = pytest.mark.gpu
+
+# (label, scheme, the fused kernel takes the last layer's last tuft)
+SHAPES = [
+    ("unaligned_512", lambda: configs.instance_area(19, 1, 16, 32), False),
+    ("unaligned_1024", lambda: configs.instance_area(51, 1, 16, 64), False),   # 16-byte windows: 2.7 M synapses
+    ("unaligned_16", lambda: configs.instance_area(33, 2, 1, 16), False),
+    ("odd_21", lambda: configs.instance_area(32, 2, 3, 7), False),
+    ("odd_24", lambda: configs.instance_area(17, 1, 1, 24), False),
+    ("single", lambda: configs.instance_area(150, 1, 1, 1), False),            # too many cells to fold into the tail
+    ("pieces_4800", lambda: configs.instance_area(11, 1, 40, 120), False),     # a cell in two pieces
+    ("one_piece_2520", lambda: configs.instance_area(12, 1, 21, 120), False),
+    ("testbed", lambda: configs.testbed_area(25), None),
+    ("mixed", lambda: configs.mixed_area(26, 38), None),
+]
+
+
+def _desc(mk, settings):
+    lmaps, areas = mk()
+    return M.area_desc("v1", lmaps, areas, settings)
+
+
+@pytest.mark.parametrize("label,mk,fused", SHAPES, ids=[s[0] for s in SHAPES])
+def test_matches_oracle(label, mk, fused):
+    ctx = cortex._Ctx(0)
+    a = cortex.CorticalArea(ctx, _desc(mk, settings_for()), 7)
+    if fused is not None:
+        last = a.plan.n_layers - 1
+        assert bool(a.tuft_form(last, a.plan.layers[last].n_tufts - 1)["fused"]) == fused
+    slab = initial_slab(a.plan, 7, scramble_seed=11)
+    a.write_slab(slab)
+    fr = frames_for(a.plan, 3, 5)
+    for k in range(3):
+        a.write_input(fr[k])
+        a.cycle(1)
+        oracle.intake(a.plan, slab, 0, 0, fr[k])
+        oracle.run(a.plan, slab, None, 1, start_cycle=k)
+        dev = a.read_slab()
+        assert np.array_equal(dev, slab), "cycle %d\n%s" % (k, diff_report(a.plan, dev, slab))
+    a.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("sides", [(19, 33, 21), (65, 71, 30)])
+def test_batched_matches_alone(sides):
+    ctx = cortex._Ctx(0)
+    descs = [_desc(lambda s=s: configs.instance_area(s, 1 + s % 2, 16, 32), settings_for()) for s in sides]
+    alone = [cortex.CorticalArea(ctx, d, 3 + k) for k, d in enumerate(descs)]
+    batched = [cortex.CorticalArea(ctx, d, 3 + k) for k, d in enumerate(descs)]
+    b = cortex.Batch(ctx, batched)
+    for c in range(4):
+        for k, (x, y) in enumerate(zip(alone, batched)):
+            f = configs.frames(1, x.input_len(), 0.05, 10 * c + k)[0]
+            x.write_input(f)
+            y.write_input(f)
+            x.cycle(1)
+        b.cycle(1)
+    for x, y in zip(alone, batched):
+        assert np.array_equal(x.read_slab(), y.read_slab())
+    b.close()
+    for a in alone + batched:
+        a.close()
+    ctx.close()
