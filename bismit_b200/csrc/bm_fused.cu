@@ -26,10 +26,16 @@
 //    the cell's lanes (redux.sync over the warp when a cell fills it).
 //
 // Gather index: each synapse's (source slice, v offset, u offset) is compiled
-// once into a 16-bit offset into the staged footprint, (slc - slc0) * TSZ +
-// v_ofs * TW + u_ofs, kept beside the synapse arrays (the canonical source
-// arrays are unchanged and remain what readback returns). The compile pass
-// runs at build and again whenever the caller writes sources or flags. A
+// once, beside the synapse arrays (the canonical source arrays are unchanged
+// and remain what readback returns): into a byte, two nibbles of offsets, and
+// 2 bits of slice where the pool has several (source_code), or, where the
+// offsets span more than 16 x 16 columns, the pool more than four slices, or
+// the general consumer serves the tuft, into a 16-bit offset into the staged
+// footprint, (slc - slc0) * TSZ + v_ofs * TW + u_ofs. Codes move 4.9 (5.1 with
+// slices) bytes a synapse in place of 5.9 for 1.5 to 3 more instructions;
+// area_256's 8 cycles 2165 -> 2010 us, 24 instances' 6 cycles 2645 -> 2602
+// (one slice only: 2053 and 2624). The compile pass runs at build and again
+// whenever the caller writes sources or flags. A
 // source it cannot express (slice outside the pool, offset beyond the pool's
 // reach -- only possible through caller writes) marks the tuft, and the
 // kernel then streams the original arrays and indexes every synapse as
@@ -57,6 +63,7 @@ constexpr int kThreads = (kWarps + 1) * 32;  // plus one producer warp
 constexpr int kMaxRecs = 8;                  // contiguous source slices served by the fast gathers
 constexpr uint32_t kMaxSmem = 110 * 1024;    // dynamic shared memory per CTA (two CTAs per SM)
 constexpr uint32_t kSmem3 = 73 * 1024;       // ... with which three CTAs fit one SM
+constexpr uint32_t kMinSmem = 32 * 1024;     // every 15-bit gather offset, even a stray one, stays inside it
 constexpr uint32_t kWaitLimit = 1u << 22;
 
 struct FusedTuftArgs {
@@ -71,6 +78,7 @@ struct FusedTuftArgs {
     uint8_t* st;
     uint8_t* fl;
     const uint16_t* gidx;   // compiled gather offsets (tiled form): bytes into the tile's footprint
+    const uint8_t* gslc;    // compact codes (at gidx): their slice plane
     uint8_t* den_act;       // tuft-relative dendrite arrays
     uint8_t* den_raw;
     uint8_t* den_st;
@@ -116,6 +124,8 @@ struct FusedTuftArgs {
     uint32_t fp_tma;                    // the footprint comes from a tensor box load (else consumers stage it)
     uint32_t ssc_soma;                  // also run ssc_cycle (spiny stellate cells of one dendrite)
     uint32_t fp_bytes;                  // bytes of that box (nrec * frows * fw)
+    uint32_t compact;                   // GatherGeo::compact
+    uint32_t code_mul;                  // footprint width / 16 - 1 (compact codes)
     uint32_t cycle_from_host;           // take the cycle number from `cycle` rather than the area's counter
     unsigned long long cycle;           // (a launch on the area's front stream, which may run ahead of the
                                         // counter: the host knows the number of the cycle it enqueues)
@@ -505,6 +515,18 @@ __device__ __forceinline__ int32_t footprint_base(const FusedTuftArgs& A, const 
            ((int32_t)((u * A.src_us) >> kSlcSclCoeffL2) - G.ulo) + (int32_t)G.xoff;
 }
 
+// Where compact codes of cell `cell` (tuft-relative) of tile G start in its
+// footprint: the cell's scaled row and column counted from the tile's first
+// cell's, i.e. its neighbourhood's corner (most negative offsets).
+__device__ __forceinline__ uint32_t code_base(const FusedTuftArgs& A, const TileGeo& G, uint32_t cell) {
+    const uint32_t local = cell - G.cell0;
+    if (A.tile_h == 1)
+        return (((G.u0 + local) * A.src_us) >> kSlcSclCoeffL2) - ((G.u0 * A.src_us) >> kSlcSclCoeffL2) + G.xoff;
+    const uint32_t q = fast_div(local, A.u_size, A.usz_magic);   // whole rows: u0 is 0
+    return ((((G.v0 + q) * A.src_vs) >> kSlcSclCoeffL2) - ((G.v0 * A.src_vs) >> kSlcSclCoeffL2)) * A.fw +
+           (((local - q * A.u_size) * A.src_us) >> kSlcSclCoeffL2) + G.xoff;
+}
+
 // syn_fire of four packed axon bytes (cl/syns.cl:2-4).
 __device__ __forceinline__ uint32_t fire4(uint32_t x) { return nz_bytes(x) | ((x >> 1) & 0x7F7F7F7Fu); }
 
@@ -756,32 +778,53 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
             if (TUFT && h == 0 && f < 4)
                 C.old |= (uint32_t)wd[(1 + f) * WIN + (off >> S_L2) - ((pos >> S_L2) & ~15u)] << 8;
         }
-        uint32_t acc = 0;
-        if (on) {
-            const uint4 str4 = *(const uint4*)(sb + 2 * SB + so);
-            const uint4 st4 = *(const uint4*)(sb + 3 * SB + so);
+        // Lanes past the tile's end gather from whatever the buffer held (any
+        // 15-bit offset, and whatever codes decode to, is inside the CTA's
+        // shared memory: kMinSmem, stray_reach) and drop the result.
+        const uint4 str4 = *(const uint4*)(sb + 2 * SB + so);
+        const uint4 st4 = *(const uint4*)(sb + 3 * SB + so);
+        const uint32_t strw[4] = {str4.x, str4.y, str4.z, str4.w};
+        const uint32_t stw[4] = {st4.x, st4.y, st4.z, st4.w};
+        uint32_t gw[8];   // footprint offsets, two a word
+        if (A.compact) {
+            const uint4 c4 = *(const uint4*)(sb + so);
+            const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w};
+            const uint32_t base = code_base(A, G, min(off, G.syn_end - 16u) >> S_L2) * 0x10001u;
+#pragma unroll
+            for (int w = 0; w < 8; w++) {
+                // (v << 4 | u) + (v << 4) * (fw / 16 - 1) = v * fw + u
+                const uint32_t x = __byte_perm(cw[w / 2], 0, (w & 1) ? 0x4342 : 0x4140);
+                gw[w] = (x & 0x00F000F0u) * A.code_mul + (x + base);
+            }
+            if (A.compact == 2) {
+                const uint32_t sl = *(const uint32_t*)(sb + SB + so / 4);
+#pragma unroll
+                for (int w = 0; w < 8; w++) gw[w] += ((sl >> (2 * w)) & 0x00030003u) * A.fsz;
+            }
+        } else {
             const uint4 g0 = *(const uint4*)(sb + 2 * so);
             const uint4 g1 = *(const uint4*)(sb + 2 * so + 16);
-            const uint32_t gw[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-            const uint32_t strw[4] = {str4.x, str4.y, str4.z, str4.w};
-            const uint32_t stw[4] = {st4.x, st4.y, st4.z, st4.w};
-            uint32_t nst[4], nfl[4], sum = 0, raw = 0;
+            const uint32_t ow[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
 #pragma unroll
-            for (int w = 0; w < 4; w++) {
-                const uint32_t lo = gw[2 * w], hi = gw[2 * w + 1];
-                nst[w] = pack4(halo[lo & 0x7FFFu], halo[(lo >> 16) & 0x7FFFu], halo[hi & 0x7FFFu],
-                               halo[(hi >> 16) & 0x7FFFu]);
-            }
+            for (int w = 0; w < 8; w++) gw[w] = ow[w] & 0x7FFF7FFFu;
+        }
+        uint32_t nst[4], nfl[4], sum = 0, raw = 0;
 #pragma unroll
-            for (int w = 0; w < 4; w++) {
-                nfl[w] = nz_bytes(stw[w]) >> 3;
-                raw = __dp4a(nst[w], 0x01010101u, raw);
-                sum = __dp4a(nst[w] & ~neg_bytes(strw[w]), 0x01010101u, sum);
-            }
+        for (int w = 0; w < 4; w++) {
+            const uint32_t lo = gw[2 * w], hi = gw[2 * w + 1];
+            nst[w] = pack4(halo[lo & 0xFFFFu], halo[lo >> 16], halo[hi & 0xFFFFu], halo[hi >> 16]);
+        }
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            nfl[w] = nz_bytes(stw[w]) >> 3;
+            raw = __dp4a(nst[w], 0x01010101u, raw);
+            sum = __dp4a(nst[w] & ~neg_bytes(strw[w]), 0x01010101u, sum);
+        }
+        if (on) {
             *(uint4*)(A.st + off) = make_uint4(nst[0], nst[1], nst[2], nst[3]);
             *(uint4*)(A.fl + off) = make_uint4(nfl[0], nfl[1], nfl[2], nfl[3]);
-            acc = (raw << 16) | sum;   // a dendrite's sums are at most 64 * 255
         }
+        uint32_t acc = (raw << 16) | sum;   // a dendrite's sums are at most 64 * 255
 #pragma unroll
         for (uint32_t m = 1; m < LPD; m <<= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, m);
         if (own) C.acc = acc;
@@ -885,7 +928,10 @@ __device__ __forceinline__ bool produce_tile(const FusedTuftArgs& A, const TileG
         const uint32_t left = G.syn_end - pos;
         const uint32_t nb = left < SB ? left : SB;
         uint8_t* dst = stages + (size_t)pb * buf_bytes;
-        uint32_t n_arr_bytes = (MODE == 0 ? 2 * nb : 3 * nb) + nb + nb + (FCLEAN ? 0 : nb);
+        // Compact codes are streamed only for the specialised consumers (MODE 0,
+        // clean flags): other modes of such a tuft run as MODE 1 (mode_of).
+        const uint32_t src_bytes = MODE != 0 ? 3 * nb : !A.compact ? 2 * nb : A.compact == 1 ? nb : nb + nb / 4;
+        uint32_t n_arr_bytes = src_bytes + nb + nb + (FCLEAN ? 0 : nb);
         // Windows of the stage's dendrites and cells, widened to 16-byte bounds.
         const uint32_t d0 = (pos >> A.spd_l2) & ~15u, d1 = (((pos + nb) >> A.spd_l2) + 15) & ~15u;
         const uint32_t c0 = (pos >> A.S_l2) & ~15u, c1 = (((pos + nb) >> A.S_l2) + 15) & ~15u;
@@ -902,7 +948,10 @@ __device__ __forceinline__ bool produce_tile(const FusedTuftArgs& A, const TileG
                 bulk_g2s(wd + 4 * A.win_bytes, A.t_st + c0, cb, &full[pb]);
             }
         }
-        if (MODE == 0) {
+        if (MODE == 0 && A.compact) {
+            bulk_g2s(dst, (const uint8_t*)A.gidx + pos, nb, &full[pb]);
+            if (A.compact == 2) bulk_g2s(dst + SB, A.gslc + pos / 4, nb / 4, &full[pb]);
+        } else if (MODE == 0) {
             bulk_g2s(dst, A.gidx + pos, 2 * nb, &full[pb]);
         } else {
             bulk_g2s(dst, A.slc + pos, nb, &full[pb]);
@@ -972,11 +1021,14 @@ __device__ __forceinline__ bool consume_tile(const FusedTuftArgs& A, const TileG
     FastCarry C = {0, kNoDen, 0};
     for (uint32_t pos = G.syn0; pos < G.syn_end; pos += SB) {
         const uint32_t cb = ring & kRingBuf;
-        bool got = !s_abort && mbar_wait(&full[cb], (ring & kRingPhase) ? 1u : 0u, A.ctl);
-        got = __all_sync(0xFFFFFFFFu, got);
-        if (!got) {
-            if (lane == 0) raise_abort(s_abort, A.ctl);
-            return false;
+        // One try first; the abort flag and the clock only while it fails.
+        if (!__all_sync(0xFFFFFFFFu, mbar_try_wait(&full[cb], (ring & kRingPhase) ? 1u : 0u))) {
+            bool got = !s_abort && mbar_wait(&full[cb], (ring & kRingPhase) ? 1u : 0u, A.ctl);
+            got = __all_sync(0xFFFFFFFFu, got);
+            if (!got) {
+                if (lane == 0) raise_abort(s_abort, A.ctl);
+                return false;
+            }
         }
         if constexpr (GEOM == 0)
             tma_stage<TUFT, MODE, FCLEAN>(A, G, halo, stages + (size_t)cb * A.stage_stride, pos, n_units_tile, lane,
@@ -1056,12 +1108,14 @@ __device__ __forceinline__ void init_ring(uint8_t* ring, uint32_t nst, volatile 
 // foreign flag bits) of a tuft, from its verification status.
 __device__ __forceinline__ uint32_t mode_of(const FusedTuftArgs& A) {
     const uint32_t status = A.ctl->tuft_status[A.status_idx];
-    return ((status & kTuftSrcOutsideTile) ? 2u : 0u) | ((status & kTuftFlagsForeign) ? 1u : 0u);
+    const uint32_t mode = ((status & kTuftSrcOutsideTile) ? 2u : 0u) | ((status & kTuftFlagsForeign) ? 1u : 0u);
+    // The general consumer reads no compact codes: foreign flags then take the
+    // original source arrays too.
+    return A.compact && mode == 1 ? 3u : mode;
 }
 
 // The general consumers out of line: inlined beside the specialised ones they
-// made the kernel spill, and with 219 KB of an SM's 228 KB taken as shared
-// memory a reload misses L1.
+// make the kernel spill.
 template <bool TUFT, int MODE, bool FCLEAN>
 __device__ __noinline__ void tma_body_general(const FusedTuftArgs& A, uint8_t* smem, volatile int& s_abort) {
     tma_body<TUFT, MODE, FCLEAN, 0>(A, smem, s_abort);
@@ -1246,6 +1300,22 @@ __global__ void k_compile_tuft(const uint8_t* __restrict__ slc, const int8_t* __
         const uint32_t* sw = (const uint32_t*)&s4;
         const uint32_t* vw = (const uint32_t*)&v4;
         const uint32_t* uw = (const uint32_t*)&u4;
+        if (g.compact) {
+            uint32_t codes[4] = {}, slices = 0;
+#pragma unroll
+            for (int b = 0; b < 16; b++) {
+                uint32_t code, k;
+                const int sh = 8 * (b & 3);
+                if (!source_code(g, (sw[b / 4] >> sh) & 0xFF, (int)(int8_t)(vw[b / 4] >> sh),
+                                 (int)(int8_t)(uw[b / 4] >> sh), code, k))
+                    bits |= kTuftSrcOutsideTile;
+                codes[b / 4] |= code << sh;
+                slices |= k << slice_shift(b);
+            }
+            *(uint4*)((uint8_t*)gidx + i) = make_uint4(codes[0], codes[1], codes[2], codes[3]);
+            if (g.compact == 2) *(uint32_t*)((uint8_t*)gidx + g.slc_off + i / 4) = slices;
+            continue;
+        }
         uint32_t out[8];
 #pragma unroll
         for (int w = 0; w < 4; w++) {
@@ -1291,6 +1361,10 @@ uint32_t ring_stages(uint64_t stride, uint64_t halo, uint32_t max_n) {
         if (128 + n * stride + halo <= kMaxSmem) return n;
     return 2;
 }
+
+// What compact codes of arbitrary bytes decode to stays below this: a base
+// inside one slice's footprint, 15 rows and columns, three slices.
+uint64_t stray_reach(uint64_t fsz, uint64_t fw) { return 4 * fsz + 16 * fw + 16; }
 
 // Largest default tile, in synapses (an explicit target may ask for more).
 constexpr uint64_t kMaxTileSyns = 65536;
@@ -1399,10 +1473,16 @@ void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int
     uint64_t fwb = (fw + 15 + 15) / 16 * 16;
     if (fwb % 32 == 0 && fwb + 16 <= 256 && (uint64_t)nrec * frows * (fwb + 16) < 32768) fwb += 16;
     tma = tma && fwb <= 256 && frows <= 256 && (uint64_t)nrec * frows * fwb < 32768;
+    // Compact codes: pools whose offsets span at most 16 x 16 columns over at
+    // most four slices; the slice plane's rows of a stage stay 16-byte aligned
+    // from 64 synapses a cell on. They need rows of a multiple of 16 bytes.
+    uint32_t compact = rv <= 7 && ru <= 7 && (nrec == 1 || (nrec <= 4 && S >= 64)) ? (nrec == 1 ? 1u : 2u) : 0u;
     if (tma) {
         fw = fwb;
     } else {
-        const uint64_t fwo = fw + (12 - fw % 8) % 8;   // fw % 8 == 4: rows an odd number of words apart
+        const uint64_t fw16 = (fw + 15) / 32 * 32 + 16;   // 16 bytes past a multiple of 32
+        if ((uint64_t)nrec * frows * fw16 >= 32768) compact = 0;
+        const uint64_t fwo = compact ? fw16 : fw + (12 - fw % 8) % 8;   // fw % 8 == 4: rows an odd number of words apart
         if ((uint64_t)nrec * frows * fwo < 32768) fw = fwo;
     }
     fsz = frows * fw;
@@ -1415,9 +1495,8 @@ void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int
     // address it with a constant base), the ring after it.
     const uint64_t ring_off = ((halo + 127) / 128) * 128;
     const uint32_t nst = ring_stages(buf_bytes, ring_off, 3);
-    // Gathers mask offsets to 15 bits: at least 32 KB of shared memory keeps
-    // every masked offset inside the CTA's allocation.
-    const uint64_t smem = std::max<uint64_t>(32768, ring_off + 128 + (uint64_t)nst * buf_bytes);
+    uint64_t smem = std::max<uint64_t>(kMinSmem, ring_off + 128 + (uint64_t)nst * buf_bytes);
+    smem = std::max(smem, stray_reach(fsz, fw));
     if (smem > kMaxSmem) return;
     FT.tiled = true;
     FT.fp_tma = tma;
@@ -1433,6 +1512,7 @@ void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int
     FT.stage_stride = buf_bytes;
     FT.win_bytes = win_bytes;
     FT.win = (T.den_idz % 16) == 0 && (T.cel_idz % 16) == 0;
+    FT.compact = consumer_shape(FT, S, spd, L.kind == BM_LYR_PYRAMIDAL) ? compact : 0u;
     FT.ring_off = (uint32_t)ring_off;
     FT.smem = (uint32_t)smem;
     FT.src_vs = vs;
@@ -1616,6 +1696,8 @@ GatherGeo geo_of(const FusedTuft& FT, const DevLayer& L, const DevTuft& T) {
     g.slc0 = FT.slc0;
     g.nrec = FT.nrec;
     g.xalign = FT.tiled && FT.fp_tma ? 1u : 0u;
+    g.compact = FT.tiled ? FT.compact : 0u;
+    g.slc_off = (uint64_t)L.cells * T.spt;
     return g;
 }
 
@@ -1667,6 +1749,7 @@ void make_args(FusedTuftArgs& A, const FusedArea& F, const uint8_t* axns, const 
     A.st = L.buf[BM_BUF_SYN_STATES] + T.syn_idz;
     A.fl = L.buf[BM_BUF_SYN_FLAG_SETS] + T.syn_idz;
     A.gidx = FT.gidx;
+    A.gslc = (const uint8_t*)FT.gidx + (uint64_t)L.cells * T.spt;
     A.den_act = L.buf[BM_BUF_DEN_ACTIVITIES] + T.den_idz;
     A.den_raw = L.buf[BM_BUF_DEN_STATES_RAW] + T.den_idz;
     A.den_st = L.buf[BM_BUF_DEN_STATES] + T.den_idz;
@@ -1729,6 +1812,8 @@ void make_args(FusedTuftArgs& A, const FusedArea& F, const uint8_t* axns, const 
         A.win_bytes = FT.win_bytes;
         A.fp_tma = FT.fp_tma ? 1u : 0u;
         A.fp_bytes = FT.nrec * FT.fsz;
+        A.compact = FT.compact;
+        A.code_mul = FT.fw / 16 - 1;
         if (FT.fp_tma) std::memcpy(&A.tmap, FT.tmap, sizeof A.tmap);
         A.geom = consumer_shape(FT, (uint32_t)S, T.spd, tuft);
     } else {
@@ -1787,16 +1872,18 @@ int prepare_fused_batch(FusedBatch& B, const std::vector<FusedJob>& jobs, const 
     for (uint32_t stride : strides) {
         std::vector<const FusedJob*> cls;
         uint32_t halo = 0;
+        uint64_t reach = kMinSmem;
         for (const FusedJob& J : jobs) {
             const FusedTuft& FT = J.F->t[J.layer][J.t];
             if (FT.stage_stride != stride) continue;
             cls.push_back(&J);
             halo = std::max(halo, ((FT.nrec * FT.fsz + 127) / 128) * 128);
+            reach = std::max(reach, stray_reach(FT.fsz, FT.fw));
         }
         uint32_t nst = ring_stages(stride, halo, shape.max_stages ? std::max<uint32_t>(2, std::min<uint32_t>(4, shape.max_stages)) : 4);
         while (nst > 2 && 128 + (uint64_t)nst * stride + halo > kMaxSmem) nst--;
         const uint64_t ring_off = halo;
-        const uint64_t smem = std::max<uint64_t>(32768, ring_off + 128 + (uint64_t)nst * stride);
+        const uint64_t smem = std::max<uint64_t>(reach, ring_off + 128 + (uint64_t)nst * stride);
         if (smem > kMaxSmem) {
             free_fused_batch(B);
             return BM_OK;

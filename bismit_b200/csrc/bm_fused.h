@@ -18,7 +18,9 @@ struct FusedTuft {
     uint32_t tile_w = 0, tile_h = 0;
     int32_t rv = 0, ru = 0;  // footprint margin: the pool's largest |v|, |u| offsets
     uint32_t fw = 0, frows = 0, fsz = 0;   // footprint width, rows, bytes per slice
-    uint16_t* gidx = nullptr;   // compiled gather offsets, one per synapse of the tuft
+    uint16_t* gidx = nullptr;   // compiled gather offsets, one per synapse of the tuft; or, with `compact`,
+                                // source codes: a byte per synapse, then the slice plane (source_code)
+    uint32_t compact = 0;       // GatherGeo::compact
     uint32_t smem = 0;       // dynamic shared memory per CTA
     uint32_t grid = 1;       // persistent grid size
     uint32_t nst = 2;        // TMA pipeline stages

@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(256) k_copy_pieces(const __grid_constant__ Cop
 // bismit's cache inserts the new key and, if that was new, drops the old one,
 // so an accepted key 0 enters unless the old key was 0, which always leaves.
 // Draws stop after kGrowMaxAttempts, keeping the last. A tiled tuft's
-// compiled gather offset follows each moved synapse. The same rule is
+// compiled gather offset (or source code) follows each moved synapse. The same rule is
 // restated in the oracle.
 __global__ void __launch_bounds__(kRegrowBlock) k_regrow(const RegrowJob* __restrict__ jobs, uint32_t n_jobs) {
     pdl_begin();
@@ -193,9 +193,22 @@ __global__ void __launch_bounds__(kRegrowBlock) k_regrow(const RegrowJob* __rest
         str[s0 + j] = (int8_t)nstr;
         // A tiled tuft's pools lie inside its footprint (every draw is held).
         if (geo.tiled) {
-            bool ok;
             const uint64_t i = s0 + j - T.syn_idz;
-            geo.gidx[i] = (uint16_t)gather_offset(geo.g, i, ns, nv, nu, ok);
+            if (geo.g.compact) {
+                uint32_t code, k;
+                source_code(geo.g, ns, nv, nu, code, k);
+                ((uint8_t*)geo.gidx)[i] = (uint8_t)code;
+                if (geo.g.compact == 2) {
+                    // Two bits of a word that other synapses share; only this
+                    // thread changes these two.
+                    uint32_t* w = (uint32_t*)((uint8_t*)geo.gidx + geo.g.slc_off) + i / 16;
+                    const uint32_t sh = slice_shift((uint32_t)i & 15u);
+                    atomicXor(w, (((*(volatile uint32_t*)w >> sh) & 3u) ^ k) << sh);
+                }
+            } else {
+                bool ok;
+                geo.gidx[i] = (uint16_t)gather_offset(geo.g, i, ns, nv, nu, ok);
+            }
         }
     }
 }

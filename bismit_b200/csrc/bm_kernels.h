@@ -54,7 +54,27 @@ struct GatherGeo {
     uint32_t fw, fsz;
     uint32_t slc0, nrec;
     uint32_t xalign;
+    // Compact codes in place of 16-bit offsets (see source_code): 0 none, 1
+    // one source slice, 2 with the slice plane, which starts slc_off bytes in.
+    uint32_t compact;
+    uint64_t slc_off;
 };
+
+// The compact form of a source: its offset in the cell's neighbourhood of up
+// to 16 x 16 columns, v in the high nibble and u in the low, both from the
+// pool's most negative offset; and its slice, counted from slc0 (2 bits, the
+// slice plane's words holding those of 16 synapses, synapse 2p at bit 2p and
+// 2p + 1 at bit 16 + 2p). Unlike a footprint offset it does not depend on the
+// tiles. False (and 0) when the footprint does not hold the source.
+__host__ __device__ __forceinline__ bool source_code(const GatherGeo& g, uint32_t slc, int vo, int uo, uint32_t& code,
+                                                     uint32_t& k) {
+    k = slc - g.slc0;
+    const bool ok = k < g.nrec && vo >= -g.rv && vo <= g.rv && uo >= -g.ru && uo <= g.ru;
+    code = ok ? (uint32_t)((vo + g.rv) << 4 | (uo + g.ru)) : 0u;
+    k = ok ? k : 0u;
+    return ok;
+}
+__host__ __device__ __forceinline__ uint32_t slice_shift(uint32_t i) { return (i & 14u) + ((i & 1u) << 4); }
 
 // The byte that the synapse at tuft offset i with source (slc, v_ofs, u_ofs)
 // gathers, as an offset into its tile's footprint; false (and 0) when the
@@ -79,7 +99,7 @@ __host__ __device__ __forceinline__ uint32_t gather_offset(const GatherGeo& g, u
 // the offsets of the synapses it moves); kept current in device memory across
 // retiling.
 struct TuftGeo {
-    uint16_t* gidx;          // null: the tuft is not tiled
+    uint16_t* gidx;          // null: the tuft is not tiled; compact codes: the code plane
     GatherGeo g;
     uint32_t tiled;
 };
