@@ -118,8 +118,8 @@ struct FusedTuftArgs {
                                         // the footprint starts at 0
     uint32_t unit_l2;                   // log2 of the bytes of one unit (chunks_per_unit * 512)
     uint32_t stage_stride;              // bytes per ring buffer (synapse arrays + windows)
-    uint32_t win;                       // dendrite / cell-tuft windows ride in the stages
-    uint32_t win_bytes;                 // bytes per window
+    uint32_t win_bytes;                 // bytes per dendrite / cell-tuft window of a stage
+    uint32_t den_mis, cel_mis;          // how far the tuft's first dendrite and cell lie past a 16-byte boundary
     uint32_t geom;                      // specialised consumer for this shape (0: the general one)
     uint32_t fp_tma;                    // the footprint comes from a tensor box load (else consumers stage it)
     uint32_t ssc_soma;                  // also run ssc_cycle (spiny stellate cells of one dendrite)
@@ -612,27 +612,23 @@ __device__ __forceinline__ void tma_stage(const FusedTuftArgs& A, const TileGeo&
         uint32_t v = 0, u = 0;
         int32_t base = 0;
         if (MODE != 0) base = footprint_base(A, G, off, v, u);
-        uint32_t act0;
-        if (A.win) {
-            // The stage carries the dendrite and cell-tuft bytes (windows start
-            // at the stage's first dendrite / cell rounded down to 16).
-            const uint8_t* wd = sb + 4 * A.stage_bytes;
-            const uint32_t lpd = 1u << A.lpd_l2;
-            act0 = (on && (lane & (lpd - 1)) == 0) ? (uint32_t)wd[(off >> A.spd_l2) - ((pos >> A.spd_l2) & ~15u)] : 0u;
-            if (TUFT && ch == 0) {
-                const uint32_t f = lane & ((1u << A.lpc_l2) - 1);
-                const uint32_t ci = (off >> A.S_l2) - ((pos >> A.S_l2) & ~15u);
-                tuft_cur = 0;
-                if (A.lpc_l2 >= 3) {
-                    if (on && f < 4) tuft_cur = wd[(1 + f) * A.win_bytes + ci];
-                } else if (on && f == 0) {
-                    tuft_cur = (uint32_t)wd[A.win_bytes + ci] | ((uint32_t)wd[2 * A.win_bytes + ci] << 8) |
-                               ((uint32_t)wd[3 * A.win_bytes + ci] << 16) | ((uint32_t)wd[4 * A.win_bytes + ci] << 24);
-                }
+        // The stage carries the dendrite and cell-tuft bytes (windows start at
+        // the stage's first dendrite / cell rounded down to 16 bytes).
+        const uint8_t* wd = sb + 4 * A.stage_bytes;
+        const uint32_t lpd = 1u << A.lpd_l2;
+        const uint32_t act0 = (on && (lane & (lpd - 1)) == 0)
+                                  ? (uint32_t)wd[A.den_mis + (off >> A.spd_l2) - ((A.den_mis + (pos >> A.spd_l2)) & ~15u)]
+                                  : 0u;
+        if (TUFT && ch == 0) {
+            const uint32_t f = lane & ((1u << A.lpc_l2) - 1);
+            const uint32_t ci = A.cel_mis + (off >> A.S_l2) - ((A.cel_mis + (pos >> A.S_l2)) & ~15u);
+            tuft_cur = 0;
+            if (A.lpc_l2 >= 3) {
+                if (on && f < 4) tuft_cur = wd[(1 + f) * A.win_bytes + ci];
+            } else if (on && f == 0) {
+                tuft_cur = (uint32_t)wd[A.win_bytes + ci] | ((uint32_t)wd[2 * A.win_bytes + ci] << 8) |
+                           ((uint32_t)wd[3 * A.win_bytes + ci] << 16) | ((uint32_t)wd[4 * A.win_bytes + ci] << 24);
             }
-        } else {
-            act0 = prefetch_act(A, off, on, lane);
-            if (ch == 0) tuft_cur = prefetch_tuft<TUFT>(A, off, on, lane);
         }
         uint4 str4{}, st4{}, fl4{}, nst4{};
         if (on) {
@@ -710,7 +706,7 @@ __host__ __device__ constexpr int geom_lpc_l2(int g) {
 // consumer) otherwise. It applies while the tuft's flags are clean and its
 // sources lie in the footprint.
 uint32_t consumer_shape(const FusedTuft& FT, uint32_t spt, uint32_t spd, bool pyramidal) {
-    if (!FT.tiled || !FT.win || spt > 1024 || FT.stage_bytes != (uint32_t)kWarps * 512 * (spt > 512 ? spt / 512 : 1))
+    if (!FT.tiled || spt > 1024 || FT.stage_bytes != (uint32_t)kWarps * 512 * (spt > 512 ? spt / 512 : 1))
         return 0;
     for (int g = 1; g < kGeoms; g++)
         if ((1u << geom_spd_l2(g)) == spd && (1u << (geom_lpc_l2(g) + 4)) == spt)
@@ -770,13 +766,14 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
         if (on && own) {
             const uint32_t den = off >> SPD_L2;
             C.den = den;
-            C.old |= wd[den - ((pos >> SPD_L2) & ~15u)];
+            C.old |= wd[A.den_mis + den - ((A.den_mis + (pos >> SPD_L2)) & ~15u)];
             // The cell's energy for the folded ssc_cycle, loaded before the
             // gathers so its latency overlaps them.
             if (!TUFT && A.ssc_soma) C.old |= (uint32_t)A.cel_en[den] << 8;
             const uint32_t f = ((uint32_t)lane & (LPCW - 1)) / LPD;
             if (TUFT && h == 0 && f < 4)
-                C.old |= (uint32_t)wd[(1 + f) * WIN + (off >> S_L2) - ((pos >> S_L2) & ~15u)] << 8;
+                C.old |= (uint32_t)wd[(1 + f) * WIN + A.cel_mis + (off >> S_L2) -
+                                      ((A.cel_mis + (pos >> S_L2)) & ~15u)] << 8;
         }
         // Lanes past the tile's end gather from whatever the buffer held (any
         // 15-bit offset, and whatever codes decode to, is inside the CTA's
@@ -932,21 +929,21 @@ __device__ __forceinline__ bool produce_tile(const FusedTuftArgs& A, const TileG
         // clean flags): other modes of such a tuft run as MODE 1 (mode_of).
         const uint32_t src_bytes = MODE != 0 ? 3 * nb : !A.compact ? 2 * nb : A.compact == 1 ? nb : nb + nb / 4;
         uint32_t n_arr_bytes = src_bytes + nb + nb + (FCLEAN ? 0 : nb);
-        // Windows of the stage's dendrites and cells, widened to 16-byte bounds.
-        const uint32_t d0 = (pos >> A.spd_l2) & ~15u, d1 = (((pos + nb) >> A.spd_l2) + 15) & ~15u;
-        const uint32_t c0 = (pos >> A.S_l2) & ~15u, c1 = (((pos + nb) >> A.S_l2) + 15) & ~15u;
-        if (A.win) n_arr_bytes += (uint32_t)(d1 - d0) + (TUFT ? 4 * (uint32_t)(c1 - c0) : 0u);
+        // Windows of the stage's dendrites and cells, widened to 16-byte bounds
+        // (counted from the boundary at or below the tuft's first one).
+        const uint32_t d0 = (A.den_mis + (pos >> A.spd_l2)) & ~15u;
+        const uint32_t db = ((A.den_mis + ((pos + nb) >> A.spd_l2) + 15) & ~15u) - d0;
+        const uint32_t c0 = (A.cel_mis + (pos >> A.S_l2)) & ~15u;
+        const uint32_t cb = ((A.cel_mis + ((pos + nb) >> A.S_l2) + 15) & ~15u) - c0;
+        n_arr_bytes += db + (TUFT ? 4 * cb : 0u);
         mbar_arrive_expect_tx(&full[pb], n_arr_bytes);
-        if (A.win) {
-            uint8_t* wd = dst + 4 * A.stage_bytes;
-            bulk_g2s(wd, A.den_act + d0, (uint32_t)(d1 - d0), &full[pb]);
-            if (TUFT) {
-                const uint32_t cb = (uint32_t)(c1 - c0);
-                bulk_g2s(wd + A.win_bytes, A.t_bid + c0, cb, &full[pb]);
-                bulk_g2s(wd + 2 * A.win_bytes, A.t_braw + c0, cb, &full[pb]);
-                bulk_g2s(wd + 3 * A.win_bytes, A.t_bst + c0, cb, &full[pb]);
-                bulk_g2s(wd + 4 * A.win_bytes, A.t_st + c0, cb, &full[pb]);
-            }
+        uint8_t* wd = dst + 4 * A.stage_bytes;
+        bulk_g2s(wd, A.den_act - A.den_mis + d0, db, &full[pb]);
+        if (TUFT) {
+            bulk_g2s(wd + A.win_bytes, A.t_bid - A.cel_mis + c0, cb, &full[pb]);
+            bulk_g2s(wd + 2 * A.win_bytes, A.t_braw - A.cel_mis + c0, cb, &full[pb]);
+            bulk_g2s(wd + 3 * A.win_bytes, A.t_bst - A.cel_mis + c0, cb, &full[pb]);
+            bulk_g2s(wd + 4 * A.win_bytes, A.t_st - A.cel_mis + c0, cb, &full[pb]);
         }
         if (MODE == 0 && A.compact) {
             bulk_g2s(dst, (const uint8_t*)A.gidx + pos, nb, &full[pb]);
@@ -1114,45 +1111,50 @@ __device__ __forceinline__ uint32_t mode_of(const FusedTuftArgs& A) {
     return A.compact && mode == 1 ? 3u : mode;
 }
 
-// The general consumers out of line: inlined beside the specialised ones they
-// make the kernel spill.
+// The general consumers beside the specialised ones are out of line: inlined
+// they make the kernel spill. Tufts whose shape has no specialised consumer
+// launch a kernel of general ones alone, with the arguments as constants
+// (through the call's pointer a 97 x 97 area's cycle was a sixth slower).
 template <bool TUFT, int MODE, bool FCLEAN>
 __device__ __noinline__ void tma_body_general(const FusedTuftArgs& A, uint8_t* smem, volatile int& s_abort) {
     tma_body<TUFT, MODE, FCLEAN, 0>(A, smem, s_abort);
 }
-template <bool TUFT>
+// FAST: the tuft's shape has a specialised consumer (A.geom).
+template <bool TUFT, bool FAST>
 __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_constant__ FusedTuftArgs A) {
     pdl_begin();
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ volatile int s_abort;   // a bounded wait gave up
     init_ring(smem + A.ring_off, A.nst, s_abort);
-    // One specialised body per gather mode and flags state (uniform per launch).
-    switch (mode_of(A)) {
-    case 0:
-        // Shapes with a specialised consumer (pyramidal tufts, or the
-        // one-dendrite cells of spiny stellates).
-        if constexpr (TUFT) {
-            switch (A.geom) {
-            case 3: tma_body<TUFT, 0, true, 3>(A, smem, s_abort); return;
-            case 4: tma_body<TUFT, 0, true, 4>(A, smem, s_abort); return;
-            case 5: tma_body<TUFT, 0, true, 5>(A, smem, s_abort); return;
-            case 6: tma_body<TUFT, 0, true, 6>(A, smem, s_abort); return;
-            case 7: tma_body<TUFT, 0, true, 7>(A, smem, s_abort); return;
-            case 8: tma_body<TUFT, 0, true, 8>(A, smem, s_abort); return;
-            default: break;
-            }
-        } else {
-            switch (A.geom) {
-            case 1: tma_body<TUFT, 0, true, 1>(A, smem, s_abort); return;
-            case 2: tma_body<TUFT, 0, true, 2>(A, smem, s_abort); return;
-            default: break;
-            }
+    // One body per gather mode and flags state (uniform per launch).
+    const uint32_t mode = mode_of(A);
+    if constexpr (!FAST) {
+        switch (mode) {
+        case 0: tma_body<TUFT, 0, true, 0>(A, smem, s_abort); break;
+        case 1: tma_body<TUFT, 0, false, 0>(A, smem, s_abort); break;
+        case 2: tma_body<TUFT, 1, true, 0>(A, smem, s_abort); break;
+        default: tma_body<TUFT, 1, false, 0>(A, smem, s_abort); break;
         }
-        tma_body_general<TUFT, 0, true>(A, smem, s_abort);
-        break;
-    case 1: tma_body_general<TUFT, 0, false>(A, smem, s_abort); break;
-    case 2: tma_body_general<TUFT, 1, true>(A, smem, s_abort); break;
-    default: tma_body_general<TUFT, 1, false>(A, smem, s_abort); break;
+        return;
+    }
+    switch (mode) {
+    case 0: break;
+    case 1: tma_body_general<TUFT, 0, false>(A, smem, s_abort); return;
+    case 2: tma_body_general<TUFT, 1, true>(A, smem, s_abort); return;
+    default: tma_body_general<TUFT, 1, false>(A, smem, s_abort); return;
+    }
+    if constexpr (TUFT) {
+        switch (A.geom) {
+        case 3: tma_body<TUFT, 0, true, 3>(A, smem, s_abort); return;
+        case 4: tma_body<TUFT, 0, true, 4>(A, smem, s_abort); return;
+        case 5: tma_body<TUFT, 0, true, 5>(A, smem, s_abort); return;
+        case 6: tma_body<TUFT, 0, true, 6>(A, smem, s_abort); return;
+        case 7: tma_body<TUFT, 0, true, 7>(A, smem, s_abort); return;
+        default: tma_body<TUFT, 0, true, 8>(A, smem, s_abort); return;
+        }
+    } else {
+        if (A.geom == 1) tma_body<TUFT, 0, true, 1>(A, smem, s_abort);
+        else tma_body<TUFT, 0, true, 2>(A, smem, s_abort);
     }
 }
 
@@ -1376,6 +1378,14 @@ int device_sms() {
     return sms;
 }
 
+// The one-tuft kernel of a layer kind, for a shape with a specialised consumer
+// or without.
+using TmaKernel = void (*)(FusedTuftArgs);
+TmaKernel tma_kernel(bool pyr, bool fast) {
+    return pyr ? (fast ? k_fused_tuft_tma<true, true> : k_fused_tuft_tma<true, false>)
+               : (fast ? k_fused_tuft_tma<false, true> : k_fused_tuft_tma<false, false>);
+}
+
 // Launch parameters of tuft t of data layer i (gidx left null). `target` is
 // the synapses per tile to aim for (0: chosen from the tuft's size);
 // `allow_tma` lets the footprint come from a tensor box load.
@@ -1487,8 +1497,8 @@ void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int
     }
     fsz = frows * fw;
     halo = (uint64_t)nrec * fsz;
-    // Windows: up to SB / 16 dendrites (or cells) per stage, widened by 16
-    // at both ends.
+    // Windows: up to SB / 16 dendrites (or cells) per stage, widened by up to
+    // 15 at both ends.
     const uint32_t win_bytes = SB / 16 + 32;
     const uint32_t buf_bytes = 4 * SB + 5 * win_bytes;
     // The footprint sits at the start of dynamic shared memory (gathers then
@@ -1511,7 +1521,6 @@ void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int
     FT.stage_bytes = SB;
     FT.stage_stride = buf_bytes;
     FT.win_bytes = win_bytes;
-    FT.win = (T.den_idz % 16) == 0 && (T.cel_idz % 16) == 0;
     FT.compact = consumer_shape(FT, S, spd, L.kind == BM_LYR_PYRAMIDAL) ? compact : 0u;
     FT.ring_off = (uint32_t)ring_off;
     FT.smem = (uint32_t)smem;
@@ -1522,7 +1531,7 @@ void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int
     for (uint32_t k = 0; k < nrec; k++) FT.src_idz[k] = P.slc_axn_idz[lo + k];
     // Persistent grid: as many CTAs as fit on the device at once.
     const bool pyr = L.kind == BM_LYR_PYRAMIDAL;
-    auto kern = pyr ? k_fused_tuft_tma<true> : k_fused_tuft_tma<false>;
+    auto kern = tma_kernel(pyr, consumer_shape(FT, S, spd, pyr) != 0);
     // The cap is a property of the kernel, shared by every area on the device:
     // set it to the largest footprint any tuft may plan, never lower.
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
@@ -1808,8 +1817,9 @@ void make_args(FusedTuftArgs& A, const FusedArea& F, const uint8_t* axns, const 
         A.ring_off = FT.ring_off;
         A.unit_l2 = 9 + ilog2(A.chunks_per_unit);
         A.stage_stride = FT.stage_stride;
-        A.win = FT.win;
         A.win_bytes = FT.win_bytes;
+        A.den_mis = (uint32_t)(T.den_idz & 15);
+        A.cel_mis = (uint32_t)(T.cel_idz & 15);
         A.fp_tma = FT.fp_tma ? 1u : 0u;
         A.fp_bytes = FT.nrec * FT.fsz;
         A.compact = FT.compact;
@@ -1834,7 +1844,7 @@ void launch_fused_tuft(const FusedArea& F, const uint8_t* axns, const SliceRec* 
     }
     const bool tuft = L.kind == BM_LYR_PYRAMIDAL;
     if (FT.tiled) {
-        auto kern = tuft ? k_fused_tuft_tma<true> : k_fused_tuft_tma<false>;
+        auto kern = tma_kernel(tuft, A.geom != 0);
         launch_pdl(kern, FT.grid, kThreads, FT.smem, s, A);
     } else {
         uint64_t want = (A.n_units + kWarps - 1) / kWarps;

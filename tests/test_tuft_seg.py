@@ -1,8 +1,8 @@
-"""The tuft kernel for shapes the tiled one does not take (bm_seg.cuh), against
-the oracle on the whole slab (tolerance: exact): synapse ranges off 16-byte
-alignment, dendrites and cells of odd lengths, cells larger than a block's
-piece, scaled and nonspatial sources, both window widths, and the batched
-form."""
+"""Tufts at odd sizes, against the oracle on the whole slab (tolerance: exact):
+the kernel for shapes the tiled one does not take (bm_seg.cuh) -- synapse
+ranges off 16-byte alignment, dendrites and cells of odd lengths, cells larger
+than a block's piece, scaled and nonspatial sources, both window widths, the
+batched form -- and the tiled one with dendrites and cells off alignment."""
 import numpy as np
 import pytest
 
@@ -22,6 +22,8 @@ SHAPES = [
     ("single", lambda: configs.instance_area(150, 1, 1, 1), False),            # too many cells to fold into the tail
     ("pieces_4800", lambda: configs.instance_area(11, 1, 40, 120), False),     # a cell in two pieces
     ("one_piece_2520", lambda: configs.instance_area(12, 1, 21, 120), False),
+    ("odd_cells", lambda: configs.benchmark_area(21, 64, 3, 16, 32, 6), True),  # dendrites and cells off alignment
+    ("odd_cells_256", lambda: configs.benchmark_area(23, 32, 3, 8, 32, 3), True),
     ("testbed", lambda: configs.testbed_area(25), None),
     ("mixed", lambda: configs.mixed_area(26, 38), None),
 ]
@@ -32,14 +34,15 @@ def _desc(mk, settings):
     return M.area_desc("v1", lmaps, areas, settings)
 
 
+@pytest.mark.parametrize("clean_flags", [False, True])
 @pytest.mark.parametrize("label,mk,fused", SHAPES, ids=[s[0] for s in SHAPES])
-def test_matches_oracle(label, mk, fused):
+def test_matches_oracle(label, mk, fused, clean_flags):
     ctx = cortex._Ctx(0)
     a = cortex.CorticalArea(ctx, _desc(mk, settings_for()), 7)
     if fused is not None:
         last = a.plan.n_layers - 1
         assert bool(a.tuft_form(last, a.plan.layers[last].n_tufts - 1)["fused"]) == fused
-    slab = initial_slab(a.plan, 7, scramble_seed=11)
+    slab = initial_slab(a.plan, 7, scramble_seed=11, clean_flags=clean_flags)
     a.write_slab(slab)
     fr = frames_for(a.plan, 3, 5)
     for k in range(3):
