@@ -309,16 +309,14 @@ void bm::exec_step(bm_area_s* A, const Step& st, cudaStream_t s, bool end_cycle)
         if (A->host_cycle % kRegrowPeriod != kRegrowPeriod - 1) break;
         run(K_REGROW, [&] { launch_regrow(A->d_regrow, (uint32_t)A->regrow.size(), A->regrow_blocks, s); });
         break;
-    case ST_SMOOTH: {
+    case ST_SMOOTH:
         // The six lattices in order (the reference runs them as one racing
         // launch; this is one of the orders it can produce).
-        const uint32_t* off = A->center_off[i][x];
-        for (int k = 0; k < 6; k++)
-            run(K_SMOOTH, [&] {
-                launch_smooth(D, A->d_centers[i][x] + off[k], off[k + 1] - off[k], (int32_t)L.ctrl[x].field_radius, s);
-            });
+        run(K_SMOOTH, [&] {
+            launch_smooth(D, A->d_centers[i][x], A->center_off[i][x], (int32_t)L.ctrl[x].field_radius, A->d_smooth, s);
+        });
+        if (own) A->launches++;   // two kernels
         break;
-    }
     case ST_FILTER: {
         // SensoryFilter::cycle (src/cortex/sensory_filter.rs:157-168) of each
         // filter in order: filter k reads its own buffer and writes the next
@@ -962,6 +960,7 @@ void free_area(bm_area_s* A) {
         dev_free(A->d_geo, pl, s);
         for (auto& row : A->d_centers)
             for (int32_t* c : row) dev_free(c, pl, s);
+        dev_free(A->d_smooth, pl, s);
         if (A->side) cudaStreamDestroy(A->side);
         if (A->ev_fork) cudaEventDestroy(A->ev_fork);
         free_front_events(A);
@@ -1227,7 +1226,8 @@ int bm_area_create(bm_ctx ctx, const bm_area_desc* desc, uint64_t seed, bm_area*
         rc = prepare_regrow(A, grow, gts);
         if (rc != BM_OK) { free_area(A); return rc; }
     }
-    // Activity smoothers' group centers.
+    // Activity smoothers' group centers, and a word per cell for their picks.
+    uint64_t smoothed = 0;
     for (uint32_t i = 0; i < A->plan.n_layers; i++) {
         const bm_layer_plan& L = A->plan.layers[i];
         for (uint32_t k = 0; k < L.n_ctrl; k++) {
@@ -1239,7 +1239,13 @@ int bm_area_create(bm_ctx ctx, const bm_area_desc* desc, uint64_t seed, bm_area*
                 e = cudaMemcpyAsync(A->d_centers[i][k], c.data(), c.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
                                     s);
             if (e != cudaSuccess) { free_area(A); return cuda_err(e, "smoother centers"); }
+            smoothed = std::max<uint64_t>(smoothed, L.cells);
         }
+    }
+    if (smoothed) {
+        e = dev_alloc(ctx, &A->d_smooth, smoothed * sizeof(uint32_t));
+        if (e == cudaSuccess) e = cudaMemsetAsync(A->d_smooth, 0, smoothed * sizeof(uint32_t), s);
+        if (e != cudaSuccess) { free_area(A); return cuda_err(e, "smoother picks"); }
     }
     for (uint32_t i = 0; i < A->plan.n_layers; i++) A->verify_pending[i] = true;
     area_steps(A, A->steps, cell_tuft_cells(A) <= kFoldCellTufts);

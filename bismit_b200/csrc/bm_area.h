@@ -220,6 +220,7 @@ struct bm_area_s {
     // lattices in center_off ranges.
     int32_t* d_centers[BM_MAX_LAYERS][BM_MAX_CTRL] = {};
     uint32_t center_off[BM_MAX_LAYERS][BM_MAX_CTRL][7] = {};
+    uint32_t* d_smooth = nullptr;   // a word per cell of the largest smoothed layer (zero between launches)
     // Per data layer, bit t: tuft t may hold source slice ids outside its
     // pool (written by the caller), so its steps may read any axon slice.
     uint8_t foreign_src[BM_MAX_LAYERS] = {};

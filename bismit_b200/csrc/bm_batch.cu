@@ -540,7 +540,7 @@ void count_launches(bm_batch_s* B) {
                 const bm_layer_plan& L = A->plan.layers[st.layer];
                 uint32_t per = 1;
                 if (st.kind == ST_TUFTS_PLAIN) per = 1 + 2 * L.n_tufts + (L.kind == BM_LYR_PYRAMIDAL ? L.n_tufts : 0);
-                if (st.kind == ST_SMOOTH) per = 6;
+                if (st.kind == ST_SMOOTH) per = 2;
                 if (st.kind == ST_FILTER) per = A->plan.filter_chains[st.idx].n_filters;
                 n += per;
             }

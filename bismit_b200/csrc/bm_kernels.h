@@ -146,8 +146,11 @@ void launch_ssc_mtp_plain(const uint8_t* axns, const DevLayer& L, const AreaCtl*
 void launch_pyr_cycle_plain(const DevLayer& L, cudaStream_t s);
 void launch_pyr_output(uint8_t* axns, const SliceRec* slices, const DevLayer& L, cudaStream_t s);
 void launch_inhib_intra_column_plain(uint8_t* axns, const SliceRec* slices, const DevLayer& L, cudaStream_t s);
-// One lattice of the activity smoother's group centers (bm_plain.cu).
-void launch_smooth(const DevLayer& L, const int32_t* centers, uint32_t n, int32_t radius, cudaStream_t s);
+// The activity smoother's six lattices of group centers, lattice k at
+// off[k] .. off[k + 1] - 1; `ops`: a zeroed word per cell of the layer, left
+// zero (bm_plain.cu).
+void launch_smooth(const DevLayer& L, const int32_t* centers, const uint32_t off[7], int32_t radius, uint32_t* ops,
+                   cudaStream_t s);
 // One retina filter (cl/filters.cl:34-100) from a (depth, v_size, u_size)
 // input grid to slices base_slc.. of `out`, each at its slice-table offset.
 void launch_retina(const uint8_t* in, uint8_t* out, const SliceRec* slices, uint32_t base_slc, uint32_t depth,

@@ -213,50 +213,94 @@ void launch_pyr_cycle_plain(const DevLayer& L, cudaStream_t s) {
 void launch_pyr_output(uint8_t* axns, const SliceRec* slices, const DevLayer& L, cudaStream_t s) {
     launch_pdl(k_pyr_output, nblk(L.cells, 256), 256, 0, s, axns, slices, L);
 }
-// smooth_activity (cl/control.cl:227-295), one lattice of group centers: each
-// center scans the hexagon of side r around it over every slice of the host
-// layer (slice, then v offset, then u offset, as the reference loops), keeps
-// the least active cell (ties: the later one) and the most active (ties: the
-// later one), then raises the least active cell's energy by one and lowers
-// the most active's by one, each within 0..255 and only when they differ.
-// The groups of one lattice do not overlap, so the centers of a launch touch
-// disjoint cells.
-__global__ void k_smooth(DevLayer L, const int32_t* __restrict__ centers, uint32_t n, int32_t r) {
+// smooth_activity (cl/control.cl:227-295). Each group center scans the hexagon
+// of side r around it over every slice of the host layer (slice, then v
+// offset, then u offset, as the reference loops), finds the least active cell
+// (ties: the later one) and the most active (ties: the later one), and raises
+// the least active cell's energy by one and lowers the most active's by one,
+// each within 0..255 and only when they differ. Six lattices of centers act
+// one after the other; within a lattice the hexagons are disjoint.
+//
+// Activities do not change while the smoother runs, so every lattice's finds
+// run at once (a warp per center), each leaving a bit per lattice at the cells
+// it picked: bit k, raise; bit 8 + k, lower. A second launch applies a cell's
+// bits in lattice order, which is what six launches one after the other do.
+// Latency-bound (a hexagon's loads, then a warp's reduction): a 120 x 120 layer
+// with r = 3 took six launches of a thread per center, 7.0 us each; the two
+// launches take SMOOTH_US (cold, ncu).
+struct SmoothRange {
+    uint32_t off[7];   // lattice k: centers off[k] .. off[k + 1] - 1
+};
+
+__global__ void __launch_bounds__(128) k_smooth_find(DevLayer L, const int32_t* __restrict__ centers, SmoothRange R,
+                                                     int32_t r, uint32_t* __restrict__ ops) {
     pdl_begin();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const uint32_t i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= R.off[6]) return;
     const int32_t cv = centers[i] >> 16, cu = (int32_t)(int16_t)(centers[i] & 0xFFFF);
     const uint8_t* act = L.buf[BM_BUF_CEL_ACTIVITIES];
-    uint8_t* en = L.buf[BM_BUF_CEL_ENERGIES];
     const int32_t vs = (int32_t)L.v_size, us = (int32_t)L.u_size;
-    uint32_t least_idx = 0, most_idx = 0;
-    uint32_t least_act = 255, most_act = 0;
+    const uint32_t side = 2 * (uint32_t)r + 1, sq = side * side;   // at most 255; sq * depth < 2^24
+    // Keys order cells by activity, then by place in the scan.
+    uint32_t least = 0xFFFFFFFFu, most = 0;
+    bool any = false;
+    auto place = [&](uint32_t p, int32_t& v, int32_t& u) {   // the p-th cell of the square around the hexagon
+        const int32_t vo = (int32_t)(p / side) - r, uo = (int32_t)(p % side) - r;
+        v = cv + vo;
+        u = cu + uo;
+        return uo >= max(-r, -vo - r) && uo <= min(r, -vo + r) && v >= 0 && v < vs && u >= 0 && u < us;
+    };
     for (uint32_t slc = 0; slc < L.depth; slc++)
-        for (int32_t vo = -r; vo <= r; vo++) {
-            const int32_t uz = max(-r, -vo - r), um = min(r, -vo + r);
-            const int32_t v = cv + vo;
-            for (int32_t uo = uz; uo <= um; uo++) {
-                const int32_t u = cu + uo;
-                if (v < 0 || v >= vs || u < 0 || u >= us) continue;
-                const uint32_t idx = slc * (uint32_t)(vs * us) + (uint32_t)(v * us + u);
-                const uint32_t a = act[idx];
-                if (a <= least_act) { least_idx = idx; least_act = a; }
-                if (a >= most_act) { most_idx = idx; most_act = a; }
-            }
+        for (uint32_t p = lane; p < sq; p += 32) {
+            int32_t v, u;
+            if (!place(p, v, u)) continue;
+            const uint32_t a = act[slc * (uint32_t)(vs * us) + (uint32_t)(v * us + u)], ord = slc * sq + p;
+            least = min(least, (a << 24) | (0xFFFFFFu - ord));
+            most = max(most, (a << 24) | ord);
+            any = true;
         }
-    // Equal indices change nothing; skipping the write matters, because a
-    // hexagon wholly outside the layer leaves both at cell 0, and writing
-    // cell 0's energy back would race the one hexagon of the lattice that
-    // holds cell 0.
-    if (least_idx == most_idx) return;
-    const uint32_t le = en[least_idx];
-    en[least_idx] = (uint8_t)(le + (uint32_t)((le < 255) & (most_act < 255)));
-    const uint32_t me = en[most_idx];
-    en[most_idx] = (uint8_t)(me - (uint32_t)((me > 0) & (most_act > 0)));
+    least = __reduce_min_sync(0xFFFFFFFFu, least);
+    most = __reduce_max_sync(0xFFFFFFFFu, most);
+    // A hexagon wholly outside the layer changes nothing, nor does one whose
+    // two cells are the same.
+    if (!__any_sync(0xFFFFFFFFu, any) || lane) return;
+    const uint32_t lo = 0xFFFFFFu - (least & 0xFFFFFFu), mo = most & 0xFFFFFFu, most_act = most >> 24;
+    if (lo == mo) return;
+    uint32_t k = 0;
+    while (i >= R.off[k + 1]) k++;
+    auto cell = [&](uint32_t ord) {
+        int32_t v, u;
+        const uint32_t slc = ord / sq;
+        place(ord - slc * sq, v, u);
+        return slc * (uint32_t)(vs * us) + (uint32_t)(v * us + u);
+    };
+    if (most_act < 255) atomicOr(&ops[cell(lo)], 1u << k);
+    if (most_act > 0) atomicOr(&ops[cell(mo)], 256u << k);
 }
 
-void launch_smooth(const DevLayer& L, const int32_t* centers, uint32_t n, int32_t radius, cudaStream_t s) {
-    if (n) launch_pdl(k_smooth, nblk(n, 128), 128, 0, s, L, centers, n, radius);
+__global__ void __launch_bounds__(128) k_smooth_apply(uint8_t* __restrict__ en, uint32_t* __restrict__ ops, uint32_t n) {
+    pdl_begin();
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n) return;
+    const uint32_t o = ops[c];
+    if (!o) return;
+    uint32_t e = en[c];
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        e += (uint32_t)(((o >> k) & 1) && e < 255);
+        e -= (uint32_t)(((o >> (8 + k)) & 1) && e > 0);
+    }
+    en[c] = (uint8_t)e;
+    ops[c] = 0;
+}
+
+void launch_smooth(const DevLayer& L, const int32_t* centers, const uint32_t off[7], int32_t radius, uint32_t* ops,
+                   cudaStream_t s) {
+    SmoothRange R;
+    for (int k = 0; k < 7; k++) R.off[k] = off[k];
+    if (!R.off[6]) return;
+    launch_pdl(k_smooth_find, nblk(R.off[6], 4), 128, 0, s, L, centers, R, radius, ops);
+    launch_pdl(k_smooth_apply, nblk(L.cells, 128), 128, 0, s, L.buf[BM_BUF_CEL_ENERGIES], ops, L.cells);
 }
 
 // retina (cl/filters.cl:34-100), one input filter over a (depth, v, u) grid

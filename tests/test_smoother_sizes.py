@@ -1,0 +1,43 @@
+"""The activity smoother's two launches against the oracle on the whole slab
+(tolerance: exact): group sides around a warp's 32 positions, layers smaller
+than a hexagon, several slices, energies at both ends of their range, batched."""
+import numpy as np
+import pytest
+
+import oracle
+from bismit_b200 import configs, cortex, map as M
+from helpers import diff_report, frames_for, initial_slab, settings_for
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("side,radius,pyr_radius", [(40, 1, 1), (33, 2, 3), (57, 3, 2), (24, 9, 7), (16, 17, 1)])
+@pytest.mark.parametrize("batched", [False, True])
+def test_sizes_match_oracle(side, radius, pyr_radius, batched):
+    ctx = cortex._Ctx(0)
+    lmaps, areas = configs.smoother_area(side, radius, pyr_radius)
+    a = cortex.CorticalArea(ctx, M.area_desc("v1", lmaps, areas, settings_for()), 7)
+    slab = initial_slab(a.plan, 7, scramble_seed=3, clean_flags=True)
+    # Energies and activities at the ends of their ranges, where the order of
+    # the six lattices shows.
+    from bismit_b200 import _ffi as F
+    rng = np.random.default_rng(side)
+    for i in range(a.plan.n_layers):
+        L = a.plan.layers[i]
+        for k in ("cel_energies", "cel_activities"):
+            off = int(L.buf_off[F.BUF[k]])
+            slab[off:off + int(L.cells)] = rng.choice([0, 0, 1, 2, 100, 254, 255, 255], int(L.cells)).astype(np.uint8)
+    a.write_slab(slab)
+    b = cortex.Batch(ctx, [a]) if batched else None
+    fr = frames_for(a.plan, 3, 5)
+    for k in range(3):
+        a.write_input(fr[k])
+        (b or a).cycle(1)
+        oracle.intake(a.plan, slab, 0, 0, fr[k])
+        oracle.run(a.plan, slab, None, 1, start_cycle=k)
+        dev = a.read_slab()
+        assert np.array_equal(dev, slab), "cycle %d\n%s" % (k, diff_report(a.plan, dev, slab))
+    if b:
+        b.close()
+    a.close()
+    ctx.close()
