@@ -123,11 +123,46 @@ bool layer_plain(const bm_area_plan& P, uint32_t i) {
     return true;
 }
 
+// Brings steps that fuse next to one another, where the order between them does
+// not show.
+//  * A smoother touches its layer's cell activities and energies only. On a
+//    pyramidal layer only a basket inhibition does too, so without one it goes
+//    ahead of the layer's tufts; on a spiny stellate layer learning does not,
+//    so it goes behind that.
+//  * A pyr_output that an inhib_intra_column of the same layer follows wrote
+//    every axon of the layer, and the intra-column step writes them all again
+//    with nothing in between reading them: it is left out.
+void order_steps(const bm_area_s* A, std::vector<Step>& v) {
+    const bm_area_plan& P = A->plan;
+    for (size_t k = 0; k < v.size(); k++) {
+        if (v[k].kind != ST_SMOOTH || P.layers[v[k].layer].kind != BM_LYR_PYRAMIDAL) continue;
+        bool basket = false;
+        for (size_t j = 0; j < k; j++)
+            basket |= v[j].layer == v[k].layer && (v[j].kind == ST_INHIB_SIMPLE || v[j].kind == ST_INHIB_PASS);
+        if (basket) continue;
+        size_t j = 0;
+        while (j < k && (v[j].layer != v[k].layer || v[j].kind == ST_SMOOTH || v[j].kind == ST_FILTER)) j++;
+        std::rotate(v.begin() + j, v.begin() + k, v.begin() + k + 1);
+    }
+    for (size_t k = v.size(); k-- > 0;) {
+        if (v[k].kind != ST_SMOOTH || P.layers[v[k].layer].kind == BM_LYR_PYRAMIDAL) continue;
+        for (size_t j = k + 1; j < v.size(); j++)
+            if (v[j].kind == ST_SSC_MTP && v[j].layer == v[k].layer) {
+                std::rotate(v.begin() + k, v.begin() + k + 1, v.begin() + j + 1);
+                break;
+            }
+    }
+    for (size_t k = 0; k + 1 < v.size(); k++)
+        if (v[k].kind == ST_PYR_OUTPUT && v[k + 1].kind == ST_INTRA_COL && v[k].layer == v[k + 1].layer)
+            v.erase(v.begin() + k);
+}
+
 // Fused forms of adjacent steps whose later stages only read what the earlier
 // ones wrote for the same cell (bm_items.cuh).
 void fuse_steps(const bm_area_s* A, std::vector<Step>& v, bool fold_cell_tufts) {
     const bm_area_plan& P = A->plan;
     std::vector<Step> out;
+    order_steps(A, v);
     for (size_t k = 0; k < v.size(); k++) {
         const Step& s = v[k];
         // A spiny stellate tuft whose cells have one dendrite also runs the

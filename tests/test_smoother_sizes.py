@@ -41,3 +41,29 @@ def test_sizes_match_oracle(side, radius, pyr_radius, batched):
         b.close()
     a.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("inhib,smooth", [(1, 2), (2, 1)])
+def test_with_basket_inhibition_on_the_pyramidal_layer(inhib, smooth):
+    """A basket inhibition writes the activities a smoother reads, whichever
+    runs first; learning follows both."""
+    ctx = cortex._Ctx(0)
+    lmaps, areas = configs.smoother_area(35, 3, 2, smoothers=False)
+    lm = lmaps["visual"]
+    lm.layer(M.LayerScheme.define("iii_inhib").cellular(
+        M.CellScheme.control(M.ControlCellKind.InhibitoryBasketSurround("iii", 3), inhib)))
+    lm.layer(M.LayerScheme.define("iii_smooth").cellular(
+        M.CellScheme.control(M.ControlCellKind.ActivitySmoother("iii", 2), smooth)))
+    a = cortex.CorticalArea(ctx, M.area_desc("v1", lmaps, areas, settings_for()), 7)
+    slab = initial_slab(a.plan, 7, scramble_seed=3, clean_flags=True)
+    a.write_slab(slab)
+    fr = frames_for(a.plan, 4, 5)
+    for k in range(4):
+        a.write_input(fr[k])
+        a.cycle(1)
+        oracle.intake(a.plan, slab, 0, 0, fr[k])
+        oracle.run(a.plan, slab, None, 1, start_cycle=k)
+        dev = a.read_slab()
+        assert np.array_equal(dev, slab), "cycle %d\n%s" % (k, diff_report(a.plan, dev, slab))
+    a.close()
+    ctx.close()
