@@ -996,6 +996,7 @@ void free_area(bm_area_s* A) {
         for (auto& row : A->d_centers)
             for (int32_t* c : row) dev_free(c, pl, s);
         dev_free(A->d_smooth, pl, s);
+        dev_free(A->d_layers, pl, s);
         if (A->side) cudaStreamDestroy(A->side);
         if (A->ev_fork) cudaEventDestroy(A->ev_fork);
         free_front_events(A);
@@ -1276,6 +1277,15 @@ int bm_area_create(bm_ctx ctx, const bm_area_desc* desc, uint64_t seed, bm_area*
             if (e != cudaSuccess) { free_area(A); return cuda_err(e, "smoother centers"); }
             smoothed = std::max<uint64_t>(smoothed, L.cells);
         }
+    }
+    bool mis = false;
+    for (uint32_t i = 0; i < A->plan.n_layers; i++)
+        for (uint32_t t = 0; t < A->plan.layers[i].n_tufts; t++) mis |= A->fused.t[i][t].ok && A->fused.t[i][t].mis;
+    if (mis) {
+        e = dev_alloc(ctx, &A->d_layers, sizeof A->dl);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(A->d_layers, A->dl, sizeof A->dl, cudaMemcpyHostToDevice, s);
+        if (e != cudaSuccess) { free_area(A); return cuda_err(e, "device layers"); }
+        A->fused.d_layers = A->d_layers;
     }
     if (smoothed) {
         e = dev_alloc(ctx, &A->d_smooth, smoothed * sizeof(uint32_t));

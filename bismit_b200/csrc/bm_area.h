@@ -164,6 +164,7 @@ struct bm_area_s {
     bool verify_pending[BM_MAX_LAYERS] = {};   // sources or flags written since the last check
     uint32_t exec_path = BM_PATH_FUSED;
     bm::FusedArea fused;
+    bm::DevLayer* d_layers = nullptr;   // dl in device memory, where an unaligned tuft may need it
     bool profiling = false;
     struct Rec { int kind; cudaEvent_t a, b; };
     std::vector<Rec> pending;

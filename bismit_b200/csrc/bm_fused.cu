@@ -53,6 +53,7 @@
 #include <new>
 
 #include "bm_kernels.h"
+#include "bm_seg.cuh"
 
 namespace bm {
 
@@ -126,6 +127,9 @@ struct FusedTuftArgs {
     uint32_t fp_bytes;                  // bytes of that box (nrec * frows * fw)
     uint32_t compact;                   // GatherGeo::compact
     uint32_t code_mul;                  // footprint width / 16 - 1 (compact codes)
+    uint32_t mis;                       // FusedTuft::mis
+    uint32_t lo_mask[4];                // the first `mis` bytes of a 16-byte window
+    const DevLayer* layer;              // the layer in device memory (mis != 0)
     uint32_t cycle_from_host;           // take the cycle number from `cycle` rather than the area's counter
     unsigned long long cycle;           // (a launch on the area's front stream, which may run ahead of the
                                         // counter: the host knows the number of the cycle it enqueues)
@@ -581,15 +585,16 @@ __device__ __forceinline__ void build_footprint(const FusedTuftArgs& A, const Ti
 // windows: MODE 0 streams gidx (2 bytes a synapse) then strength, state and
 // (unless FCLEAN) flags; MODE 1 streams slc, v_ofs, u_ofs, strength, state,
 // flags. The common form (MODE 0, FCLEAN) takes SB synapses a stage; the wider
-// forms take SB / 2, so every form fits the same buffer.
+// forms take SB / 2, so every form fits the same buffer. MODE 2 is MODE 0 for
+// tufts whose synapses start off a 16-byte boundary: arrays of SB + 16.
 template <int MODE, bool FCLEAN>
 __device__ __forceinline__ uint32_t stage_syns(uint32_t SB) {
-    return (MODE == 0 && FCLEAN) ? SB : SB / 2;
+    return (MODE != 1 && FCLEAN) ? SB : SB / 2;
 }
 template <int MODE>
 __device__ __forceinline__ uint32_t arr_off(int which, uint32_t SB) {
     // which: 0 strength, 1 state, 2 flags
-    return MODE == 0 ? (2 + which) * SB : (3 + which) * SB;
+    return MODE != 1 ? (2 + which) * SB : (3 + which) * SB;
 }
 
 // Consumer work of one stage: this warp's unit (a chunk, or a cell of
@@ -701,17 +706,20 @@ __host__ __device__ constexpr int geom_lpc_l2(int g) {
 
 }  // namespace
 
-// The specialised consumer a tiled tuft's launches dispatch to: shapes 3..7
-// on pyramidal layers, 1..2 on spiny stellate layers, 0 (the general
-// consumer) otherwise. It applies while the tuft's flags are clean and its
-// sources lie in the footprint.
-uint32_t consumer_shape(const FusedTuft& FT, uint32_t spt, uint32_t spd, bool pyramidal) {
-    if (!FT.tiled || spt > 1024 || FT.stage_bytes != (uint32_t)kWarps * 512 * (spt > 512 ? spt / 512 : 1))
-        return 0;
+// The specialised consumer of cells of spt synapses in dendrites of spd:
+// shapes 3..8 on pyramidal layers, 1..2 on spiny stellate layers, 0 (the
+// general consumer) otherwise.
+static uint32_t fast_shape(uint32_t spt, uint32_t spd, bool pyramidal) {
     for (int g = 1; g < kGeoms; g++)
         if ((1u << geom_spd_l2(g)) == spd && (1u << (geom_lpc_l2(g) + 4)) == spt)
             return (pyramidal ? g >= 3 : g <= 2) ? (uint32_t)g : 0u;
     return 0;
+}
+
+// The one a tiled tuft's launches dispatch to. It applies while the tuft's
+// flags are clean and its sources lie in the footprint.
+uint32_t consumer_shape(const FusedTuft& FT, uint32_t spt, uint32_t spd, bool pyramidal) {
+    return FT.tiled ? fast_shape(spt, spd, pyramidal) : 0u;
 }
 
 namespace {
@@ -736,7 +744,14 @@ constexpr uint32_t kNoDen = 0xFFFFFFFFu;
 
 // Consumer work of one stage: new states and flags of this warp's unit, and
 // its dendrites' sums into C.
-template <bool TUFT, int SPD_L2, int LPC_L2>
+// With MIS the synapses start `mis` bytes past a 16-byte boundary. A lane then
+// takes a window of the arrays' own alignment: `mis` synapses of the 16 before
+// its own and 16 - mis of its own, whose other sums come from the next lane.
+// The two windows that a unit shares with its neighbours (the first one's tail
+// and the one past the last's head, 16 bytes together) are taken a byte a lane.
+// 12 cycles of a 150 x 150 x 3 instance with 16 x 64 tufts: 2906 us in the
+// windowed form (bm_seg.cuh), 1247 us here.
+template <bool TUFT, int SPD_L2, int LPC_L2, bool MIS>
 __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo& G, const uint8_t* halo,
                                            const uint8_t* sb, uint32_t pos, int lane, int wib, FastCarry& C) {
     // A cell of 1024 synapses (LPC_L2 == 6) is taken as two units of 512; its
@@ -745,6 +760,7 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
     constexpr uint32_t HALVES = LPC_L2 == 6 ? 2u : 1u;
     constexpr uint32_t UNIT = 512u * HALVES;             // synapses of a warp per stage
     constexpr uint32_t SB = kWarps * UNIT;
+    constexpr uint32_t SX = SB + (MIS ? 16 : 0);         // bytes of a 1-byte array in the stage
     constexpr uint32_t WIN = SB / 16 + 32;
     constexpr uint32_t LPD = 1u << (SPD_L2 - 4);
     constexpr uint32_t LPC = 1u << LPC_L2;               // lanes a cell spans over its halves
@@ -756,7 +772,7 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
         C.old += HALVES * kCarryUnit;
         return;
     }
-    const uint8_t* wd = sb + 4 * SB;
+    const uint8_t* wd = sb + 4 * SX;
 #pragma unroll 1
     for (uint32_t h = 0; h < HALVES; h++, C.old += kCarryUnit) {
         const uint32_t so = (uint32_t)wib * UNIT + h * 512u + (uint32_t)lane * 16;
@@ -778,15 +794,17 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
         // Lanes past the tile's end gather from whatever the buffer held (any
         // 15-bit offset, and whatever codes decode to, is inside the CTA's
         // shared memory: kMinSmem, stray_reach) and drop the result.
-        const uint4 str4 = *(const uint4*)(sb + 2 * SB + so);
-        const uint4 st4 = *(const uint4*)(sb + 3 * SB + so);
+        const uint4 str4 = *(const uint4*)(sb + 2 * SX + so);
+        const uint4 st4 = *(const uint4*)(sb + 3 * SX + so);
         const uint32_t strw[4] = {str4.x, str4.y, str4.z, str4.w};
         const uint32_t stw[4] = {st4.x, st4.y, st4.z, st4.w};
         uint32_t gw[8];   // footprint offsets, two a word
+        uint32_t edge_base = 0;
         if (A.compact) {
             const uint4 c4 = *(const uint4*)(sb + so);
             const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w};
-            const uint32_t base = code_base(A, G, min(off, G.syn_end - 16u) >> S_L2) * 0x10001u;
+            const uint32_t base1 = code_base(A, G, min(off, G.syn_end - 16u) >> S_L2), base = base1 * 0x10001u;
+            if (MIS) edge_base = base1;
 #pragma unroll
             for (int w = 0; w < 8; w++) {
                 // (v << 4 | u) + (v << 4) * (fw / 16 - 1) = v * fw + u
@@ -794,7 +812,7 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
                 gw[w] = (x & 0x00F000F0u) * A.code_mul + (x + base);
             }
             if (A.compact == 2) {
-                const uint32_t sl = *(const uint32_t*)(sb + SB + so / 4);
+                const uint32_t sl = *(const uint32_t*)(sb + SX + so / 4);
 #pragma unroll
                 for (int w = 0; w < 8; w++) gw[w] += ((sl >> (2 * w)) & 0x00030003u) * A.fsz;
             }
@@ -805,7 +823,7 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
 #pragma unroll
             for (int w = 0; w < 8; w++) gw[w] = ow[w] & 0x7FFF7FFFu;
         }
-        uint32_t nst[4], nfl[4], sum = 0, raw = 0;
+        uint32_t nst[4], nfl[4], sum = 0, raw = 0, sum_lo = 0, raw_lo = 0;
 #pragma unroll
         for (int w = 0; w < 4; w++) {
             const uint32_t lo = gw[2 * w], hi = gw[2 * w + 1];
@@ -814,12 +832,48 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
 #pragma unroll
         for (int w = 0; w < 4; w++) {
             nfl[w] = nz_bytes(stw[w]) >> 3;
+            const uint32_t pos4 = nst[w] & ~neg_bytes(strw[w]);
             raw = __dp4a(nst[w], 0x01010101u, raw);
-            sum = __dp4a(nst[w] & ~neg_bytes(strw[w]), 0x01010101u, sum);
+            sum = __dp4a(pos4, 0x01010101u, sum);
+            if (MIS) {
+                raw_lo = __dp4a(nst[w] & A.lo_mask[w], 0x01010101u, raw_lo);
+                sum_lo = __dp4a(pos4 & A.lo_mask[w], 0x01010101u, sum_lo);
+            }
         }
-        if (on) {
-            *(uint4*)(A.st + off) = make_uint4(nst[0], nst[1], nst[2], nst[3]);
-            *(uint4*)(A.fl + off) = make_uint4(nfl[0], nfl[1], nfl[2], nfl[3]);
+        if (on && (!MIS || lane > 0)) {
+            const uint32_t w0 = off - (MIS ? A.mis : 0u);
+            *(uint4*)(A.st + w0) = make_uint4(nst[0], nst[1], nst[2], nst[3]);
+            *(uint4*)(A.fl + w0) = make_uint4(nfl[0], nfl[1], nfl[2], nfl[3]);
+        }
+        if constexpr (MIS) {
+            const uint32_t u0 = (uint32_t)wib * UNIT + h * 512u;           // the unit in the stage
+            const uint32_t n_on = min(32u, (G.syn_end - (pos + u0)) >> 4);   // its lanes inside the tile
+            uint32_t edge = 0;
+            if (lane < 16) {
+                const bool head = (uint32_t)lane < A.mis;   // of the window past the last
+                const uint32_t e = u0 + (head ? n_on * 16 : 0u) + (uint32_t)lane;
+                uint32_t o;
+                if (A.compact) {
+                    const uint32_t c = sb[e];
+                    o = edge_base + (c >> 4) * A.fw + (c & 15u);
+                    if (A.compact == 2)
+                        o += ((*(const uint32_t*)(sb + SX + (e & ~15u) / 4) >> slice_shift(e & 15u)) & 3u) * A.fsz;
+                } else {
+                    o = *(const uint16_t*)(sb + 2 * e) & 0x7FFFu;
+                }
+                const uint32_t a = halo[o];
+                const uint32_t i = pos + e - A.mis;
+                A.st[i] = (uint8_t)a;
+                A.fl[i] = sb[3 * SX + e] ? kSynPrevActiveFlag : (uint8_t)0;
+                if (head) edge = (a << 16) | ((int8_t)sb[2 * SX + e] >= 0 ? a : 0u);
+            }
+            const uint32_t lo = (raw_lo << 16) | sum_lo;
+            const uint32_t past = __reduce_add_sync(0xFFFFFFFFu, edge), next = __shfl_down_sync(0xFFFFFFFFu, lo, 1);
+            // Of this lane's own 16 synapses: its window's without the first
+            // `mis`, and the next window's first `mis`.
+            const uint32_t t = ((raw << 16) | sum) - lo + ((uint32_t)lane + 1 == n_on ? past : next);
+            raw = t >> 16;
+            sum = t & 0xFFFFu;
         }
         uint32_t acc = (raw << 16) | sum;   // a dendrite's sums are at most 64 * 255
 #pragma unroll
@@ -927,8 +981,12 @@ __device__ __forceinline__ bool produce_tile(const FusedTuftArgs& A, const TileG
         uint8_t* dst = stages + (size_t)pb * buf_bytes;
         // Compact codes are streamed only for the specialised consumers (MODE 0,
         // clean flags): other modes of such a tuft run as MODE 1 (mode_of).
-        const uint32_t src_bytes = MODE != 0 ? 3 * nb : !A.compact ? 2 * nb : A.compact == 1 ? nb : nb + nb / 4;
-        uint32_t n_arr_bytes = src_bytes + nb + nb + (FCLEAN ? 0 : nb);
+        // MODE 2 copies the 16-byte windows the stage's synapses touch: one
+        // more than they would fill, from the boundary below the first.
+        const uint32_t nw = nb + (MODE == 2 ? 16 : 0), SX = SB + (MODE == 2 ? 16 : 0);
+        const uint32_t plane = MODE == 2 ? nb / 4 + 16 : nb / 4;
+        const uint32_t src_bytes = MODE == 1 ? 3 * nb : !A.compact ? 2 * nw : A.compact == 1 ? nw : nw + plane;
+        uint32_t n_arr_bytes = src_bytes + nw + nw + (FCLEAN ? 0 : nb);
         // Windows of the stage's dendrites and cells, widened to 16-byte bounds
         // (counted from the boundary at or below the tuft's first one).
         const uint32_t d0 = (A.den_mis + (pos >> A.spd_l2)) & ~15u;
@@ -937,7 +995,7 @@ __device__ __forceinline__ bool produce_tile(const FusedTuftArgs& A, const TileG
         const uint32_t cb = ((A.cel_mis + ((pos + nb) >> A.S_l2) + 15) & ~15u) - c0;
         n_arr_bytes += db + (TUFT ? 4 * cb : 0u);
         mbar_arrive_expect_tx(&full[pb], n_arr_bytes);
-        uint8_t* wd = dst + 4 * A.stage_bytes;
+        uint8_t* wd = dst + 4 * (A.stage_bytes + (MODE == 2 ? 16 : 0));
         bulk_g2s(wd, A.den_act - A.den_mis + d0, db, &full[pb]);
         if (TUFT) {
             bulk_g2s(wd + A.win_bytes, A.t_bid - A.cel_mis + c0, cb, &full[pb]);
@@ -945,18 +1003,19 @@ __device__ __forceinline__ bool produce_tile(const FusedTuftArgs& A, const TileG
             bulk_g2s(wd + 3 * A.win_bytes, A.t_bst - A.cel_mis + c0, cb, &full[pb]);
             bulk_g2s(wd + 4 * A.win_bytes, A.t_st - A.cel_mis + c0, cb, &full[pb]);
         }
-        if (MODE == 0 && A.compact) {
-            bulk_g2s(dst, (const uint8_t*)A.gidx + pos, nb, &full[pb]);
-            if (A.compact == 2) bulk_g2s(dst + SB, A.gslc + pos / 4, nb / 4, &full[pb]);
-        } else if (MODE == 0) {
-            bulk_g2s(dst, A.gidx + pos, 2 * nb, &full[pb]);
+        if (MODE != 1 && A.compact) {
+            bulk_g2s(dst, (const uint8_t*)A.gidx + pos, nw, &full[pb]);
+            if (A.compact == 2) bulk_g2s(dst + SX, A.gslc + pos / 4, plane, &full[pb]);
+        } else if (MODE != 1) {
+            bulk_g2s(dst, A.gidx + pos, 2 * nw, &full[pb]);
         } else {
             bulk_g2s(dst, A.slc + pos, nb, &full[pb]);
             bulk_g2s(dst + SB, A.vofs + pos, nb, &full[pb]);
             bulk_g2s(dst + 2 * SB, A.uofs + pos, nb, &full[pb]);
         }
-        bulk_g2s(dst + arr_off<MODE>(0, SB), A.str + pos, nb, &full[pb]);
-        bulk_g2s(dst + arr_off<MODE>(1, SB), A.st + pos, nb, &full[pb]);
+        const uint32_t mis = MODE == 2 ? A.mis : 0u;
+        bulk_g2s(dst + arr_off<MODE>(0, SX), A.str - mis + pos, nw, &full[pb]);
+        bulk_g2s(dst + arr_off<MODE>(1, SX), A.st - mis + pos, nw, &full[pb]);
         if (!FCLEAN) bulk_g2s(dst + arr_off<MODE>(2, SB), A.fl + pos, nb, &full[pb]);
         if (++pb == nst) { pb = 0; ps.pround++; }
     }
@@ -1031,7 +1090,7 @@ __device__ __forceinline__ bool consume_tile(const FusedTuftArgs& A, const TileG
             tma_stage<TUFT, MODE, FCLEAN>(A, G, halo, stages + (size_t)cb * A.stage_stride, pos, n_units_tile, lane,
                                           wib, rnd);
         else
-            stage_fast<TUFT, geom_spd_l2(GEOM), geom_lpc_l2(GEOM)>(A, G, halo, stages + (size_t)cb * A.stage_stride,
+            stage_fast<TUFT, geom_spd_l2(GEOM), geom_lpc_l2(GEOM), MODE == 2>(A, G, halo, stages + (size_t)cb * A.stage_stride,
                                                                    pos, lane, wib, C);
         // The buffer is released after the finish: released before it, the
         // loads run further ahead and the cycle is slower (area_256 0.296 ms
@@ -1051,6 +1110,24 @@ __device__ __forceinline__ bool consume_tile(const FusedTuftArgs& A, const TileG
 // Shared-memory barriers of a CTA: the ring's full[nst] and empty[nst], then
 // the footprint's at a fixed slot (nst <= 4).
 constexpr uint32_t kFpFullSlot = 8;
+
+// An unaligned tuft whose flags have foreign bits or whose sources lie outside
+// the footprint: the consumer warps take tile G's cells in the windowed form
+// (bm_seg.cuh), its shared memory where the footprint would be.
+struct ConsumerSync {
+    static __device__ __forceinline__ void sync() { consumers_sync(); }
+};
+constexpr uint32_t kSegBytes = (sizeof(SegSmem) + 127) / 128 * 128;
+__device__ __noinline__ void seg_tile(const FusedTuftArgs& A, uint32_t t, uint8_t* smem, int32_t rnd) {
+    const TileGeo G = tile_geo(A, t);
+    const uint32_t c1 = G.cell0 + G.h * G.w, per = seg_cells(1u << A.S_l2, 16);
+    for (uint32_t c0 = G.cell0; c0 < c1; c0 += per) {
+        tuft_seg_block<16, kWarps * 32, ConsumerSync>(A.axns, A.slices, *A.layer, A.status_idx % BM_MAX_TUFTS, rnd, c0,
+                                                      min(per, c1 - c0), false, *(SegSmem*)smem);
+        consumers_sync();
+    }
+    fence_proxy_async_smem();   // a later tile's box may overwrite these bytes
+}
 
 template <bool TUFT, int MODE, bool FCLEAN, int GEOM>
 __device__ __forceinline__ void tma_body(const FusedTuftArgs& A, uint8_t* smem, volatile int& s_abort) {
@@ -1119,8 +1196,9 @@ template <bool TUFT, int MODE, bool FCLEAN>
 __device__ __noinline__ void tma_body_general(const FusedTuftArgs& A, uint8_t* smem, volatile int& s_abort) {
     tma_body<TUFT, MODE, FCLEAN, 0>(A, smem, s_abort);
 }
-// FAST: the tuft's shape has a specialised consumer (A.geom).
-template <bool TUFT, bool FAST>
+// FORM: 0 the tuft's shape has no specialised consumer (A.geom), 1 it has, 2 it
+// has and the tuft is unaligned.
+template <bool TUFT, int FORM>
 __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_constant__ FusedTuftArgs A) {
     pdl_begin();
     extern __shared__ __align__(128) uint8_t smem[];
@@ -1128,7 +1206,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_con
     init_ring(smem + A.ring_off, A.nst, s_abort);
     // One body per gather mode and flags state (uniform per launch).
     const uint32_t mode = mode_of(A);
-    if constexpr (!FAST) {
+    if constexpr (FORM == 0) {
         switch (mode) {
         case 0: tma_body<TUFT, 0, true, 0>(A, smem, s_abort); break;
         case 1: tma_body<TUFT, 0, false, 0>(A, smem, s_abort); break;
@@ -1137,6 +1215,15 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_con
         }
         return;
     }
+    constexpr int M = FORM == 2 ? 2 : 0;
+    if constexpr (FORM == 2) {
+        if (mode) {
+            if (threadIdx.x >= kWarps * 32) return;
+            const int32_t rnd = rnd_at(A.rnd_key, cycle_of(A));
+            for (uint32_t t = blockIdx.x; t < A.n_tiles; t += gridDim.x) seg_tile(A, t, smem, rnd);
+            return;
+        }
+    } else
     switch (mode) {
     case 0: break;
     case 1: tma_body_general<TUFT, 0, false>(A, smem, s_abort); return;
@@ -1145,12 +1232,12 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_con
     }
     if constexpr (TUFT) {
         switch (A.geom) {
-        case 3: tma_body<TUFT, 0, true, 3>(A, smem, s_abort); return;
-        case 4: tma_body<TUFT, 0, true, 4>(A, smem, s_abort); return;
-        case 5: tma_body<TUFT, 0, true, 5>(A, smem, s_abort); return;
-        case 6: tma_body<TUFT, 0, true, 6>(A, smem, s_abort); return;
-        case 7: tma_body<TUFT, 0, true, 7>(A, smem, s_abort); return;
-        default: tma_body<TUFT, 0, true, 8>(A, smem, s_abort); return;
+        case 3: tma_body<TUFT, M, true, 3>(A, smem, s_abort); return;
+        case 4: tma_body<TUFT, M, true, 4>(A, smem, s_abort); return;
+        case 5: tma_body<TUFT, M, true, 5>(A, smem, s_abort); return;
+        case 6: tma_body<TUFT, M, true, 6>(A, smem, s_abort); return;
+        case 7: tma_body<TUFT, M, true, 7>(A, smem, s_abort); return;
+        default: tma_body<TUFT, M, true, 8>(A, smem, s_abort); return;
         }
     } else {
         if (A.geom == 1) tma_body<TUFT, 0, true, 1>(A, smem, s_abort);
@@ -1187,7 +1274,8 @@ __device__ __forceinline__ uint32_t job_of(const BatchParams& P, uint32_t t) {
     return lo;
 }
 
-template <bool TUFT>
+// MIS: every job is an unaligned tuft.
+template <bool TUFT, bool MIS>
 __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_batch(const __grid_constant__ BatchParams P) {
     pdl_begin();
     extern __shared__ __align__(128) uint8_t smem[];
@@ -1223,6 +1311,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_batch(const __grid_c
             }
             const TileGeo G = tile_geo(A, t - P.tile0[j]);
             bool ok;
+            if constexpr (MIS) {
+                if (mode) continue;   // no stages: the consumers take the tile in the windowed form
+                ok = produce_tile<TUFT, 2, true>(A, G, stages, full, empty, ps, s_abort);
+            } else
             switch (mode) {
             case 0: ok = produce_tile<TUFT, 0, true>(A, G, stages, full, empty, ps, s_abort); break;
             case 1: ok = produce_tile<TUFT, 0, false>(A, G, stages, full, empty, ps, s_abort); break;
@@ -1251,6 +1343,17 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_batch(const __grid_c
         const TileGeo G = tile_geo(A, t - P.tile0[j]);
 #define BM_CONSUME(M, FC, GM)                                                                                   \
     ok = consume_tile<TUFT, M, FC, GM>(A, G, halo, stages, full, empty, fp_full, ring, lane, wib, rnd, s_abort)
+        if constexpr (MIS) {
+            if (mode) continue;   // taken below
+            switch (A.geom) {
+            case 3: BM_CONSUME(2, true, 3); break;
+            case 4: BM_CONSUME(2, true, 4); break;
+            case 5: BM_CONSUME(2, true, 5); break;
+            case 6: BM_CONSUME(2, true, 6); break;
+            case 7: BM_CONSUME(2, true, 7); break;
+            default: BM_CONSUME(2, true, 8); break;
+            }
+        } else
         switch (mode) {
         case 0:
             if constexpr (TUFT) {
@@ -1277,64 +1380,72 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_batch(const __grid_c
         }
 #undef BM_CONSUME
     }
+    if constexpr (MIS) {
+        // The tiles of tufts that need the windowed form, after the others:
+        // with the call in the loop above its state would be spilled.
+        if (consumers_sync_or(!ok || s_abort)) return;
+        for (uint32_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+            const uint32_t j = job_of(P, t);
+            const FusedTuftArgs& A = P.jobs[j];
+            if (mode_of(A)) seg_tile(A, t - P.tile0[j], smem, rnd_at(A.rnd_key, cycle_of(A)));   // ends on a barrier
+        }
+    }
 }
 
 // ------------------------------------------------------ source compile ----
 // Writes each synapse's gather offset into its tile's footprint
 // (gather_offset) and sets kTuftSrcOutsideTile if a source cannot be served
 // from the footprint, kTuftFlagsForeign if a flag byte has bits other than
-// SYN_PREV_ACTIVE. 16 synapses (of one cell) per thread. With gidx == nullptr
-// (untiled tufts) only the flags are checked.
+// SYN_PREV_ACTIVE. A 16-byte window per thread. With gidx == nullptr (untiled
+// tufts) only the flags are checked.
+// The arrays are given from the 16-byte boundary at or below the tuft's first
+// synapse (g.pad before it), and so are the compiled data.
 __global__ void k_compile_tuft(const uint8_t* __restrict__ slc, const int8_t* __restrict__ vo,
                                const int8_t* __restrict__ uo, const uint8_t* __restrict__ fl, uint16_t* gidx,
                                uint64_t n, GatherGeo g, unsigned int* status) {
     pdl_begin();
     uint32_t bits = 0;
-    for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * 16; i < n;
+    for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * 16; i < n + g.pad;
          i += (uint64_t)gridDim.x * blockDim.x * 16) {
+        // The window's synapses of this tuft.
+        const uint32_t b0 = i < g.pad ? g.pad : 0u, b1 = i + 16 > n + g.pad ? (uint32_t)(n + g.pad - i) : 16u;
+        auto mine = [&](uint32_t b) { return b >= b0 && b < b1; };
         const uint4 f4 = *(const uint4*)(fl + i);
-        const uint32_t* fw4 = (const uint32_t*)&f4;
+        const uint32_t fw4[4] = {f4.x, f4.y, f4.z, f4.w};
 #pragma unroll
-        for (int w = 0; w < 4; w++)
-            if (fw4[w] & 0xEFEFEFEFu) bits |= kTuftFlagsForeign;
+        for (int b = 0; b < 16; b++)
+            if (mine(b) && ((fw4[b / 4] >> (8 * (b & 3))) & 0xEFu)) bits |= kTuftFlagsForeign;
         if (!gidx) continue;
         const uint4 s4 = *(const uint4*)(slc + i), v4 = *(const uint4*)(vo + i), u4 = *(const uint4*)(uo + i);
-        const uint32_t* sw = (const uint32_t*)&s4;
-        const uint32_t* vw = (const uint32_t*)&v4;
-        const uint32_t* uw = (const uint32_t*)&u4;
-        if (g.compact) {
-            uint32_t codes[4] = {}, slices = 0;
+        const uint32_t sw[4] = {s4.x, s4.y, s4.z, s4.w};
+        const uint32_t vw[4] = {v4.x, v4.y, v4.z, v4.w};
+        const uint32_t uw[4] = {u4.x, u4.y, u4.z, u4.w};
+        uint32_t codes[4] = {}, slices = 0, out[8] = {};
 #pragma unroll
-            for (int b = 0; b < 16; b++) {
+        for (int b = 0; b < 16; b++) {
+            if (!mine(b)) continue;
+            const int sh = 8 * (b & 3);
+            const uint32_t sl = (sw[b / 4] >> sh) & 0xFF;
+            const int v = (int)(int8_t)(vw[b / 4] >> sh), u = (int)(int8_t)(uw[b / 4] >> sh);
+            bool ok;
+            if (g.compact) {
                 uint32_t code, k;
-                const int sh = 8 * (b & 3);
-                if (!source_code(g, (sw[b / 4] >> sh) & 0xFF, (int)(int8_t)(vw[b / 4] >> sh),
-                                 (int)(int8_t)(uw[b / 4] >> sh), code, k))
-                    bits |= kTuftSrcOutsideTile;
+                ok = source_code(g, sl, v, u, code, k);
                 codes[b / 4] |= code << sh;
                 slices |= k << slice_shift(b);
+            } else {
+                out[b / 2] |= gather_offset(g, i + b - g.pad, sl, v, u, ok) << (16 * (b & 1));
             }
+            if (!ok) bits |= kTuftSrcOutsideTile;
+        }
+        if (g.compact) {
             *(uint4*)((uint8_t*)gidx + i) = make_uint4(codes[0], codes[1], codes[2], codes[3]);
             if (g.compact == 2) *(uint32_t*)((uint8_t*)gidx + g.slc_off + i / 4) = slices;
-            continue;
+        } else {
+            uint4* dst = (uint4*)(gidx + i);
+            dst[0] = make_uint4(out[0], out[1], out[2], out[3]);
+            dst[1] = make_uint4(out[4], out[5], out[6], out[7]);
         }
-        uint32_t out[8];
-#pragma unroll
-        for (int w = 0; w < 4; w++) {
-            uint32_t o[4];
-#pragma unroll
-            for (int b = 0; b < 4; b++) {
-                bool ok;
-                o[b] = gather_offset(g, i, (sw[w] >> (8 * b)) & 0xFF, (int)(int8_t)(vw[w] >> (8 * b)),
-                                     (int)(int8_t)(uw[w] >> (8 * b)), ok);
-                if (!ok) bits |= kTuftSrcOutsideTile;
-            }
-            out[2 * w] = o[0] | (o[1] << 16);
-            out[2 * w + 1] = o[2] | (o[3] << 16);
-        }
-        uint4* dst = (uint4*)(gidx + i);
-        dst[0] = make_uint4(out[0], out[1], out[2], out[3]);
-        dst[1] = make_uint4(out[4], out[5], out[6], out[7]);
     }
     bits = __reduce_or_sync(0xFFFFFFFFu, bits);
     if ((threadIdx.x & 31) == 0 && bits) atomicOr(status, bits);
@@ -1379,18 +1490,18 @@ int device_sms() {
 }
 
 // The one-tuft kernel of a layer kind, for a shape with a specialised consumer
-// or without.
+// or without, or for an unaligned tuft.
 using TmaKernel = void (*)(FusedTuftArgs);
-TmaKernel tma_kernel(bool pyr, bool fast) {
-    return pyr ? (fast ? k_fused_tuft_tma<true, true> : k_fused_tuft_tma<true, false>)
-               : (fast ? k_fused_tuft_tma<false, true> : k_fused_tuft_tma<false, false>);
+TmaKernel tma_kernel(bool pyr, bool fast, bool mis) {
+    if (pyr) return mis ? k_fused_tuft_tma<true, 2> : fast ? k_fused_tuft_tma<true, 1> : k_fused_tuft_tma<true, 0>;
+    return fast ? k_fused_tuft_tma<false, 1> : k_fused_tuft_tma<false, 0>;
 }
 
 // Launch parameters of tuft t of data layer i (gidx left null). `target` is
 // the synapses per tile to aim for (0: chosen from the tuft's size);
 // `allow_tma` lets the footprint come from a tensor box load.
-void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int sms, uint32_t target_syns = 0,
-               bool allow_tma = true) {
+void plan_tuft_form(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int sms, uint32_t target_syns,
+                    bool allow_tma) {
     const bm_layer_plan& L = P.layers[i];
     bool aligned = true;
     for (int k = 0; k < BM_BUF_COUNT; k++)
@@ -1398,7 +1509,11 @@ void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int
     const bm_tuft_plan& T = L.tufts[t];
     FT = FusedTuft{};
     uint32_t spd = T.syns_per_den, dpt = T.dens_per_tft;
-    FT.ok = aligned && pow2(spd) && spd >= 16 && spd <= 512 && pow2(dpt) && (T.syn_idz % 16) == 0;
+    // Off a 16-byte boundary only the specialised pyramidal consumers serve a
+    // tuft (plan_tuft gives it up again if it does not come out tiled).
+    FT.mis = (uint32_t)(T.syn_idz % 16);
+    FT.ok = aligned && pow2(spd) && spd >= 16 && spd <= 512 && pow2(dpt) &&
+            (!FT.mis || (L.kind == BM_LYR_PYRAMIDAL && fast_shape(T.syns_per_tft, spd, true)));
     // Fast gathers serve the pool's distinct slices when their ids are
     // contiguous and spatial (mid 0, where bismit's scalar and vec4 index
     // forms agree); anything else takes the general per-synapse path.
@@ -1487,6 +1602,7 @@ void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int
     // most four slices; the slice plane's rows of a stage stay 16-byte aligned
     // from 64 synapses a cell on. They need rows of a multiple of 16 bytes.
     uint32_t compact = rv <= 7 && ru <= 7 && (nrec == 1 || (nrec <= 4 && S >= 64)) ? (nrec == 1 ? 1u : 2u) : 0u;
+    if (FT.mis && S < 512) compact = 0;   // an unaligned window then reaches over two cells
     if (tma) {
         fw = fwb;
     } else {
@@ -1500,10 +1616,10 @@ void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int
     // Windows: up to SB / 16 dendrites (or cells) per stage, widened by up to
     // 15 at both ends.
     const uint32_t win_bytes = SB / 16 + 32;
-    const uint32_t buf_bytes = 4 * SB + 5 * win_bytes;
+    const uint32_t buf_bytes = 4 * (SB + (FT.mis ? 16 : 0)) + 5 * win_bytes;
     // The footprint sits at the start of dynamic shared memory (gathers then
     // address it with a constant base), the ring after it.
-    const uint64_t ring_off = ((halo + 127) / 128) * 128;
+    const uint64_t ring_off = std::max<uint64_t>(((halo + 127) / 128) * 128, FT.mis ? kSegBytes : 0);
     const uint32_t nst = ring_stages(buf_bytes, ring_off, 3);
     uint64_t smem = std::max<uint64_t>(kMinSmem, ring_off + 128 + (uint64_t)nst * buf_bytes);
     smem = std::max(smem, stray_reach(fsz, fw));
@@ -1531,7 +1647,7 @@ void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int
     for (uint32_t k = 0; k < nrec; k++) FT.src_idz[k] = P.slc_axn_idz[lo + k];
     // Persistent grid: as many CTAs as fit on the device at once.
     const bool pyr = L.kind == BM_LYR_PYRAMIDAL;
-    auto kern = tma_kernel(pyr, consumer_shape(FT, S, spd, pyr) != 0);
+    auto kern = tma_kernel(pyr, consumer_shape(FT, S, spd, pyr) != 0, FT.mis != 0);
     // The cap is a property of the kernel, shared by every area on the device:
     // set it to the largest footprint any tuft may plan, never lower.
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
@@ -1542,6 +1658,14 @@ void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int
     FT.grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(n_tiles, (uint64_t)sms * std::max(per_sm, 1)));
 }
 
+}  // namespace
+
+namespace {
+void plan_tuft(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t, int sms, uint32_t target_syns = 0,
+               bool allow_tma = true) {
+    plan_tuft_form(FT, P, i, t, sms, target_syns, allow_tma);
+    if (FT.mis && !FT.tiled) FT.ok = false;
+}
 }  // namespace
 
 int plan_fused(FusedArea& F, const bm_area_plan& P) {
@@ -1584,6 +1708,10 @@ bool retile_fused_tuft(FusedArea& F, const bm_area_plan& P, uint32_t layer, uint
     return true;
 }
 
+// Bytes of the compiled data of an unaligned tuft of n synapses: offsets or
+// codes, with room for the windows its stages copy past its end.
+static uint64_t gidx_bytes(uint64_t n) { return 2 * n + 256; }
+
 int prepare_fused(FusedArea& F, const bm_area_plan& P, std::string* err) {
     int rc = plan_fused(F, P);
     if (rc != BM_OK) return rc;
@@ -1593,9 +1721,9 @@ int prepare_fused(FusedArea& F, const bm_area_plan& P, std::string* err) {
             FusedTuft& FT = F.t[i][t];
             if (!FT.tiled) continue;
             const uint64_t n_syn = (uint64_t)P.layers[i].cells * P.layers[i].tufts[t].syns_per_tft;
-            const cudaError_t e = F.pool ? cudaMallocFromPoolAsync((void**)&FT.gidx, n_syn * sizeof(int16_t), F.pool,
-                                                                   F.pool_stream)
-                                         : cudaMalloc(&FT.gidx, n_syn * sizeof(int16_t));
+            const uint64_t bytes = FT.mis ? gidx_bytes(n_syn) : n_syn * sizeof(int16_t);
+            const cudaError_t e = F.pool ? cudaMallocFromPoolAsync((void**)&FT.gidx, bytes, F.pool, F.pool_stream)
+                                         : cudaMalloc(&FT.gidx, bytes);
             if (e != cudaSuccess) {
                 cudaGetLastError();
                 FT.gidx = nullptr;
@@ -1689,6 +1817,8 @@ void free_fused(FusedArea& F, cudaStream_t s) {
 
 namespace {
 
+// Where the slice plane starts behind the codes of n synapses, `pad` in.
+uint64_t slice_plane_off(uint64_t n, uint32_t pad) { return pad ? (n + 32 + 15) / 16 * 16 : n; }
 GatherGeo geo_of(const FusedTuft& FT, const DevLayer& L, const DevTuft& T) {
     GatherGeo g{};
     g.S_l2 = (uint32_t)ilog2(T.spt);
@@ -1706,7 +1836,8 @@ GatherGeo geo_of(const FusedTuft& FT, const DevLayer& L, const DevTuft& T) {
     g.nrec = FT.nrec;
     g.xalign = FT.tiled && FT.fp_tma ? 1u : 0u;
     g.compact = FT.tiled ? FT.compact : 0u;
-    g.slc_off = (uint64_t)L.cells * T.spt;
+    g.pad = FT.mis;
+    g.slc_off = slice_plane_off((uint64_t)L.cells * T.spt, FT.mis);
     return g;
 }
 
@@ -1726,13 +1857,12 @@ void launch_compile_tuft(const FusedArea& F, const DevLayer& L, uint32_t layer, 
     unsigned int* status = &ctl->tuft_status[layer * BM_MAX_TUFTS + t];
     cudaMemsetAsync(status, 0, sizeof(unsigned int), s);
     const uint64_t n = (uint64_t)L.cells * T.spt;
-    const uint64_t threads = (n + 15) / 16;
+    const uint64_t threads = (n + FT.mis + 15) / 16;
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((threads + 255) / 256, (uint64_t)F.sms * 8));
-    launch_pdl(k_compile_tuft, grid, 256, 0, s, L.buf[BM_BUF_SYN_SRC_SLC_IDS] + T.syn_idz,
-                                        (const int8_t*)L.buf[BM_BUF_SYN_SRC_COL_V_OFFS] + T.syn_idz,
-                                        (const int8_t*)L.buf[BM_BUF_SYN_SRC_COL_U_OFFS] + T.syn_idz,
-                                        L.buf[BM_BUF_SYN_FLAG_SETS] + T.syn_idz, FT.tiled ? FT.gidx : nullptr, n,
-                                        geo_of(FT, L, T), status);
+    const uint64_t z = T.syn_idz - FT.mis;
+    launch_pdl(k_compile_tuft, grid, 256, 0, s, L.buf[BM_BUF_SYN_SRC_SLC_IDS] + z,
+               (const int8_t*)L.buf[BM_BUF_SYN_SRC_COL_V_OFFS] + z, (const int8_t*)L.buf[BM_BUF_SYN_SRC_COL_U_OFFS] + z,
+               L.buf[BM_BUF_SYN_FLAG_SETS] + z, FT.tiled ? FT.gidx : nullptr, n, geo_of(FT, L, T), status);
 }
 
 void launch_verify_tufts(const FusedArea& F, const DevLayer& L, uint32_t layer, AreaCtl* ctl, cudaStream_t s) {
@@ -1758,7 +1888,10 @@ void make_args(FusedTuftArgs& A, const FusedArea& F, const uint8_t* axns, const 
     A.st = L.buf[BM_BUF_SYN_STATES] + T.syn_idz;
     A.fl = L.buf[BM_BUF_SYN_FLAG_SETS] + T.syn_idz;
     A.gidx = FT.gidx;
-    A.gslc = (const uint8_t*)FT.gidx + (uint64_t)L.cells * T.spt;
+    A.gslc = (const uint8_t*)FT.gidx + slice_plane_off((uint64_t)L.cells * T.spt, FT.mis);
+    A.mis = FT.mis;
+    for (uint32_t k = 0; k < FT.mis; k++) A.lo_mask[k / 4] |= 0xFFu << (8 * (k & 3));
+    A.layer = F.d_layers ? F.d_layers + layer : nullptr;
     A.den_act = L.buf[BM_BUF_DEN_ACTIVITIES] + T.den_idz;
     A.den_raw = L.buf[BM_BUF_DEN_STATES_RAW] + T.den_idz;
     A.den_st = L.buf[BM_BUF_DEN_STATES] + T.den_idz;
@@ -1844,7 +1977,7 @@ void launch_fused_tuft(const FusedArea& F, const uint8_t* axns, const SliceRec* 
     }
     const bool tuft = L.kind == BM_LYR_PYRAMIDAL;
     if (FT.tiled) {
-        auto kern = tma_kernel(tuft, A.geom != 0);
+        auto kern = tma_kernel(tuft, A.geom != 0, FT.mis != 0);
         launch_pdl(kern, FT.grid, kThreads, FT.smem, s, A);
     } else {
         uint64_t want = (A.n_units + kWarps - 1) / kWarps;
@@ -1858,6 +1991,13 @@ void launch_fused_tuft(const FusedArea& F, const uint8_t* axns, const SliceRec* 
 }
 
 // ---------------------------------------------------------- batched form --
+namespace {
+using BatchKernel = void (*)(BatchParams);
+BatchKernel batch_kernel(bool pyr, bool mis) {
+    return pyr ? (mis ? k_fused_tuft_batch<true, true> : k_fused_tuft_batch<true, false>) : k_fused_tuft_batch<false, false>;
+}
+}  // namespace
+
 int prepare_fused_batch(FusedBatch& B, const std::vector<FusedJob>& jobs, const BatchShape& shape) {
     free_fused_batch(B);
     B = FusedBatch{};
@@ -1869,10 +2009,9 @@ int prepare_fused_batch(FusedBatch& B, const std::vector<FusedJob>& jobs, const 
         if (!FT.ok || !FT.tiled || !FT.gidx || (J.L->kind == BM_LYR_PYRAMIDAL) != tuft) return BM_OK;
         sms = (uint32_t)J.F->sms;
     }
-    auto kern = tuft ? k_fused_tuft_batch<true> : k_fused_tuft_batch<false>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
     // Jobs of one stage geometry share launches (a launch's ring is uniform,
-    // and jobs with smaller stages then keep three CTAs per SM).
+    // and jobs with smaller stages then keep three CTAs per SM). Unaligned
+    // tufts' stages are a little larger: they get launches of their own.
     std::vector<uint32_t> strides;
     for (const FusedJob& J : jobs) {
         const uint32_t st = J.F->t[J.layer][J.t].stage_stride;
@@ -1881,15 +2020,20 @@ int prepare_fused_batch(FusedBatch& B, const std::vector<FusedJob>& jobs, const 
     std::sort(strides.begin(), strides.end());
     for (uint32_t stride : strides) {
         std::vector<const FusedJob*> cls;
+        bool mis = false;
         uint32_t halo = 0;
         uint64_t reach = kMinSmem;
         for (const FusedJob& J : jobs) {
             const FusedTuft& FT = J.F->t[J.layer][J.t];
             if (FT.stage_stride != stride) continue;
             cls.push_back(&J);
+            mis = FT.mis != 0;
             halo = std::max(halo, ((FT.nrec * FT.fsz + 127) / 128) * 128);
             reach = std::max(reach, stray_reach(FT.fsz, FT.fw));
         }
+        if (mis) halo = std::max(halo, kSegBytes);
+        const BatchKernel kern = batch_kernel(tuft, mis);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
         uint32_t nst = ring_stages(stride, halo, shape.max_stages ? std::max<uint32_t>(2, std::min<uint32_t>(4, shape.max_stages)) : 4);
         while (nst > 2 && 128 + (uint64_t)nst * stride + halo > kMaxSmem) nst--;
         const uint64_t ring_off = halo;
@@ -1928,6 +2072,7 @@ int prepare_fused_batch(FusedBatch& B, const std::vector<FusedJob>& jobs, const 
             B.params.push_back(P);
             B.grids.push_back((uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(total, (uint64_t)sms * std::max(per_sm, 1))));
             B.smems.push_back((uint32_t)smem);
+            B.mis.push_back(mis);
             B.n_tiles += total;
         }
     }
@@ -1941,9 +2086,8 @@ uint32_t fused_batch_stages(const void* params) { return ((const BatchParams*)pa
 
 void launch_fused_batch(const FusedBatch& B, cudaStream_t s) {
     if (!B.ok || !B.n_tiles) return;
-    auto kern = B.tuft ? k_fused_tuft_batch<true> : k_fused_tuft_batch<false>;
     for (size_t k = 0; k < B.params.size(); k++)
-        launch_pdl(kern, B.grids[k], kThreads, B.smems[k], s, *(const BatchParams*)B.params[k]);
+        launch_pdl(batch_kernel(B.tuft, B.mis[k] != 0), B.grids[k], kThreads, B.smems[k], s, *(const BatchParams*)B.params[k]);
 }
 
 void free_fused_batch(FusedBatch& B) {
@@ -1951,6 +2095,7 @@ void free_fused_batch(FusedBatch& B) {
     B.params.clear();
     B.grids.clear();
     B.smems.clear();
+    B.mis.clear();
     B.ok = false;
 }
 

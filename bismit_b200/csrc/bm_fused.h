@@ -21,6 +21,8 @@ struct FusedTuft {
     uint16_t* gidx = nullptr;   // compiled gather offsets, one per synapse of the tuft; or, with `compact`,
                                 // source codes: a byte per synapse, then the slice plane (source_code)
     uint32_t compact = 0;       // GatherGeo::compact
+    uint32_t mis = 0;           // the synapses start this far past a 16-byte boundary (pyramidal shapes with a
+                                // specialised consumer only)
     uint32_t smem = 0;       // dynamic shared memory per CTA
     uint32_t grid = 1;       // persistent grid size
     uint32_t nst = 2;        // TMA pipeline stages
@@ -49,10 +51,13 @@ struct FusedArea {
     // pool_stream when set, else cudaMalloc.
     cudaMemPool_t pool = nullptr;
     cudaStream_t pool_stream = nullptr;
+    const DevLayer* d_layers = nullptr;   // the area's layers in device memory (read by unaligned tufts whose
+                                          // flags or sources take the windowed form)
 };
 
 // Decides, per tuft, whether the fused kernel applies (syns_per_den a power of
-// two in 16..512, dens_per_tft a power of two, 16-byte aligned ranges) and
+// two in 16..512, dens_per_tft a power of two, synapses 16-byte aligned unless
+// the shape has a specialised pyramidal consumer) and
 // its gather form. Tufts that do not qualify run the plain per-stage kernels.
 int prepare_fused(FusedArea& F, const bm_area_plan& P, std::string* err);
 // The same decisions without allocating (gidx pointers left null), for every
@@ -108,6 +113,7 @@ struct FusedBatch {
     std::vector<void*> params;   // host parameter blocks, one launch each (up to 80 jobs of one
     std::vector<uint32_t> grids; // stage geometry per launch)
     std::vector<uint32_t> smems;
+    std::vector<uint8_t> mis;    // launch k's jobs are unaligned tufts
     uint32_t n_jobs = 0, n_tiles = 0;
 };
 // Launch shape of a batched tuft step, as the autotuner sets it: the ring's

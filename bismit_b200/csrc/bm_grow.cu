@@ -193,21 +193,21 @@ __global__ void __launch_bounds__(kRegrowBlock) k_regrow(const RegrowJob* __rest
         str[s0 + j] = (int8_t)nstr;
         // A tiled tuft's pools lie inside its footprint (every draw is held).
         if (geo.tiled) {
-            const uint64_t i = s0 + j - T.syn_idz;
+            const uint64_t i = s0 + j - T.syn_idz, at = i + geo.g.pad;
             if (geo.g.compact) {
                 uint32_t code, k;
                 source_code(geo.g, ns, nv, nu, code, k);
-                ((uint8_t*)geo.gidx)[i] = (uint8_t)code;
+                ((uint8_t*)geo.gidx)[at] = (uint8_t)code;
                 if (geo.g.compact == 2) {
                     // Two bits of a word that other synapses share; only this
                     // thread changes these two.
-                    uint32_t* w = (uint32_t*)((uint8_t*)geo.gidx + geo.g.slc_off) + i / 16;
-                    const uint32_t sh = slice_shift((uint32_t)i & 15u);
+                    uint32_t* w = (uint32_t*)((uint8_t*)geo.gidx + geo.g.slc_off) + at / 16;
+                    const uint32_t sh = slice_shift((uint32_t)at & 15u);
                     atomicXor(w, (((*(volatile uint32_t*)w >> sh) & 3u) ^ k) << sh);
                 }
             } else {
                 bool ok;
-                geo.gidx[i] = (uint16_t)gather_offset(geo.g, i, ns, nv, nu, ok);
+                geo.gidx[at] = (uint16_t)gather_offset(geo.g, i, ns, nv, nu, ok);
             }
         }
     }

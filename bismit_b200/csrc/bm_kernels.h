@@ -58,6 +58,9 @@ struct GatherGeo {
     // one source slice, 2 with the slice plane, which starts slc_off bytes in.
     uint32_t compact;
     uint64_t slc_off;
+    // The tuft's synapses start `pad` bytes past a 16-byte boundary: compiled
+    // data are kept at synapse + pad, so they lie as the synapse arrays do.
+    uint32_t pad;
 };
 
 // The compact form of a source: its offset in the cell's neighbourhood of up

@@ -1,9 +1,8 @@
 // bm_seg.cuh -- one tuft's stages for tufts the fused tuft kernel does not
 // take: dendrites whose length is no power of two in 16..512 (one synapse, 8,
-// 12, 24, ...), dendrite counts that are no power of two, and tufts whose
-// synapses do not start on a 16-byte boundary (any tuft behind one whose
-// synapse count is no multiple of 16, as on a 150 x 150 grid behind a
-// one-synapse tuft).
+// 12, 24, ...), dendrite counts that are no power of two, and, of tufts whose
+// synapses do not start on a 16-byte boundary, those the tiled kernel's
+// unaligned form does not serve.
 //
 // A block takes whole cells, in pieces of whole dendrites of at most
 // kSegSyns synapses, in three steps:
@@ -18,7 +17,8 @@
 // The gathers with their source extraction and bounds checks bound it. A
 // thread per cell, the form it replaces, walked the cell's synapses one by
 // one: the 16 x 64 tuft of a 150 x 150 x 3 layer (69 M synapses, 8 bytes off
-// alignment) took 3.43 ms and takes 0.236 ms; 27,648 cells of 4 x 8 dendrites
+// alignment) took 3.43 ms and 0.236 ms this way (the tiled kernel's unaligned
+// form: 0.092); 27,648 cells of 4 x 8 dendrites
 // 23.2 us, now 10.1; 30,000 cells of 4 x 12 with nonspatial sources 44 us,
 // now 15.3 (cold, ncu).
 #pragma once
@@ -52,8 +52,13 @@ template <int W> struct SegVec;
 template <> struct SegVec<16> { using T = uint4; };
 template <> struct SegVec<4> { using T = uint32_t; };
 
-// Cells [c0, c0 + nc) of tuft t; every thread of a block of kSegBlock calls it.
-template <int W>
+struct SegBlockSync {
+    static __device__ __forceinline__ void sync() { __syncthreads(); }
+};
+
+// Cells [c0, c0 + nc) of tuft t (at most seg_cells of them), by NT threads
+// (threadIdx.x < NT) that Sync::sync() joins.
+template <int W, uint32_t NT = kSegBlock, class Sync = SegBlockSync>
 __device__ __forceinline__ void tuft_seg_block(const uint8_t* __restrict__ axns, const SliceRec* __restrict__ slices,
                                                const DevLayer& L, uint32_t t, int32_t rnd, uint32_t c0, uint32_t nc,
                                                bool soma, SegSmem& S) {
@@ -67,7 +72,7 @@ __device__ __forceinline__ void tuft_seg_block(const uint8_t* __restrict__ axns,
     // axon alone; any other slice id takes the general index.
     const SliceRec r0 = slices[T.src_slc];
     const uint32_t sv = r0.y & 0xFFFFu, su = r0.y >> 16, vs = r0.z & 0xFFu, us = (r0.z >> 8) & 0xFFu;
-    for (uint32_t k = tid; k < 256; k += kSegBlock) {
+    for (uint32_t k = tid; k < 256; k += NT) {
         uint32_t x = 0xFFFFFFFFu;
         if (k < L.n_slices) {
             const SliceRec r = slices[k];
@@ -75,7 +80,7 @@ __device__ __forceinline__ void tuft_seg_block(const uint8_t* __restrict__ axns,
         }
         S.sx[k] = x;
     }
-    __syncthreads();
+    Sync::sync();
     const uint8_t* a_slc = L.buf[BM_BUF_SYN_SRC_SLC_IDS];
     const uint8_t* a_vo = L.buf[BM_BUF_SYN_SRC_COL_V_OFFS];
     const uint8_t* a_uo = L.buf[BM_BUF_SYN_SRC_COL_U_OFFS];
@@ -88,7 +93,7 @@ __device__ __forceinline__ void tuft_seg_block(const uint8_t* __restrict__ axns,
         const uint32_t nd = min(d_step, d_end - d0);
         const uint64_t lo = T.syn_idz + (uint64_t)d0 * spd, hi = lo + (uint64_t)nd * spd;
         const uint64_t base = lo & ~15ull;
-        for (uint64_t g = base + (uint64_t)tid * W; g < hi; g += (uint64_t)kSegBlock * W) {
+        for (uint64_t g = base + (uint64_t)tid * W; g < hi; g += (uint64_t)NT * W) {
             if (W < 16 && g + W <= lo) continue;
             const V slc_v = *(const V*)(a_slc + g), vo_v = *(const V*)(a_vo + g), uo_v = *(const V*)(a_uo + g);
             const V str_v = *(const V*)(a_str + g), st_v = *(const V*)(a_st + g), fl_v = *(const V*)(a_fl + g);
@@ -161,9 +166,9 @@ __device__ __forceinline__ void tuft_seg_block(const uint8_t* __restrict__ axns,
                     }
             }
         }
-        __syncthreads();
+        Sync::sync();
         // den_cycle_tft, cl/bismit.cl:695-747.
-        for (uint32_t k = tid; k < nd; k += kSegBlock) {
+        for (uint32_t k = tid; k < nd; k += NT) {
             const uint32_t d = d0 + k;
             const uint64_t di = T.den_idz + d;
             const uint8_t act0 = L.buf[BM_BUF_DEN_ACTIVITIES][di];
@@ -191,10 +196,10 @@ __device__ __forceinline__ void tuft_seg_block(const uint8_t* __restrict__ axns,
             S.draw[d - d_first] = (uint8_t)d_raw;
             S.dst[d - d_first] = (uint8_t)d_st;
         }
-        __syncthreads();
+        Sync::sync();
     }
     if (L.kind != BM_LYR_PYRAMIDAL) return;
-    for (uint32_t k = tid; k < nc; k += kSegBlock) tft_cycle_of(L, T, c0 + k, S.draw + k * dpt, S.dst + k * dpt);
+    for (uint32_t k = tid; k < nc; k += NT) tft_cycle_of(L, T, c0 + k, S.draw + k * dpt, S.dst + k * dpt);
 }
 
 }  // namespace bm

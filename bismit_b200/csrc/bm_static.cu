@@ -171,7 +171,7 @@ extern "C" int bm_tuft_cycle_static(const bm_area_plan* plan, uint32_t layer, ui
     plan_fused_tuft(F, P, layer, tuft);
     bind_fused_tuft(F, P, layer, tuft, (const uint8_t*)slab + P.axon_off);
     FusedTuft& FT = F.t[layer][tuft];
-    if (!FT.ok)
+    if (!FT.ok || FT.mis)
         return set_err(BM_ERR_UNSUPPORTED,
                        "bm_tuft_cycle_static: tuft %u of layer %u is outside the fused kernel's shapes "
                        "(syns_per_den a power of two in 16..512, dens_per_tft a power of two, 16-byte aligned buffers)",

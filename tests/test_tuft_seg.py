@@ -7,15 +7,23 @@ import numpy as np
 import pytest
 
 import oracle
-from bismit_b200 import configs, cortex, map as M
+from bismit_b200 import _ffi as F, configs, cortex, map as M
 from helpers import diff_report, frames_for, initial_slab, settings_for
 
 pytestmark = pytest.mark.gpu
 
 # (label, scheme, the fused kernel takes the last layer's last tuft)
 SHAPES = [
-    ("unaligned_512", lambda: configs.instance_area(19, 1, 16, 32), False),
-    ("unaligned_1024", lambda: configs.instance_area(51, 1, 16, 64), False),   # 16-byte windows: 2.7 M synapses
+    ("unaligned_512", lambda: configs.instance_area(19, 1, 16, 32), True),
+    ("unaligned_1024", lambda: configs.instance_area(51, 1, 16, 64), True),
+    # Every specialised shape, at odd offsets, several slices and ragged rows.
+    ("unaligned_128", lambda: configs.instance_area(23, 2, 8, 16), True),
+    ("unaligned_256a", lambda: configs.instance_area(21, 3, 16, 16), True),
+    ("unaligned_256b", lambda: configs.instance_area(27, 1, 8, 32), True),
+    ("unaligned_512b", lambda: configs.instance_area(29, 3, 8, 64), True),
+    ("unaligned_512c", lambda: configs.instance_area(66, 4, 16, 32), True),
+    ("unaligned_1024b", lambda: configs.instance_area(37, 3, 16, 64), True),
+    ("wide_16", lambda: configs.instance_area(321, 3, 1, 8), False),           # 16-byte windows
     ("unaligned_16", lambda: configs.instance_area(33, 2, 1, 16), False),
     ("odd_21", lambda: configs.instance_area(32, 2, 3, 7), False),
     ("odd_24", lambda: configs.instance_area(17, 1, 1, 24), False),
@@ -75,4 +83,44 @@ def test_batched_matches_alone(sides):
     b.close()
     for a in alone + batched:
         a.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("shape", [(19, 1, 16, 32), (37, 3, 16, 64), (23, 2, 8, 16)])
+@pytest.mark.parametrize("batched", [False, True])
+def test_unaligned_sources_moved(shape, batched):
+    """Regrowth moves sources of an unaligned tuft (its compiled codes and
+    offsets follow), then the caller writes sources past the pool's reach (the
+    tuft takes the windowed form) and back."""
+    ctx = cortex._Ctx(0)
+    a = cortex.CorticalArea(ctx, _desc(lambda: configs.instance_area(*shape), settings_for("regrowth")), 7)
+    slab = initial_slab(a.plan, 7, scramble_seed=11, clean_flags=True)
+    a.write_slab(slab)
+    a.set_cycle(199)
+    b = cortex.Batch(ctx, [a]) if batched else None
+    fr = frames_for(a.plan, 5, 5)
+
+    def step(k):
+        a.write_input(fr[k])
+        (b or a).cycle(1)
+        oracle.intake(a.plan, slab, 0, 0, fr[k])
+        oracle.run(a.plan, slab, None, 1, start_cycle=199 + k)
+        dev = a.read_slab()
+        assert np.array_equal(dev, slab), "cycle %d\n%s" % (199 + k, diff_report(a.plan, dev, slab))
+
+    for k in range(3):   # fires in the cycle numbered 200
+        step(k)
+    last = a.plan.n_layers - 1
+    off = int(a.plan.layers[last].buf_off[F.BUF["syn_src_col_v_offs"]])
+    n = int(a.plan.layers[last].n_syns)
+    keep = slab[off:off + n].copy()
+    slab[off + n - 700:off + n:3] = 100
+    a.write("syn_src_col_v_offs", slab[off:off + n].view(np.int8), layer=last)
+    step(3)
+    slab[off:off + n] = keep
+    a.write("syn_src_col_v_offs", keep.view(np.int8), layer=last)
+    step(4)
+    if b:
+        b.close()
+    a.close()
     ctx.close()
