@@ -551,6 +551,7 @@ int schedule_front(bm_area_s* A, const std::vector<StepAccess>& acc) {
     A->intake_prev.clear();
     A->intake_readers.clear();
     A->main_ev_needed.clear();
+    A->front_ev_needed.clear();
     A->front_ax_w.reset();
     size_t f = 0;
     if (A->exec_path == BM_PATH_FUSED)
@@ -562,24 +563,66 @@ int schedule_front(bm_area_s* A, const std::vector<StepAccess>& acc) {
     A->front_prev.assign(f, {});
     A->front_waits.assign(n, {});
     A->main_ev_needed.assign(n, 0);
+    A->front_ev_needed.assign(f, 0);
     A->intake_readers.assign(n, 0);
     for (size_t k = 0; k < f; k++) A->front_ax_w |= acc[k].ax_w;
-    const StepAccess in = intake_access(A->plan);
-    for (size_t t = f; t < n; t++) {
-        const bool counter_only = A->steps[t].kind == ST_CYCLE_END;
-        for (size_t k = 0; k < f; k++) {
-            if (!counter_only && conflict(acc[t], acc[k])) {
-                A->front_prev[k].push_back(t);
-                if (!A->step_side[t]) A->main_ev_needed[t] = 1;
-            }
-            if (conflict(acc[k], acc[t])) A->front_waits[t].push_back(k);
-        }
-        if (!counter_only && conflict(in, acc[t])) {
-            A->intake_prev.push_back(t);
-            if (!A->step_side[t]) A->main_ev_needed[t] = 1;
-            A->intake_readers[t] = 1;
+    // With the front stream in use a side step pays only if some main step
+    // runs beside it: between it and the first step that waits for it.
+    A->front_fork = false;
+    for (size_t k = f; k < n; k++) {
+        if (!A->step_side[k]) continue;
+        for (size_t t = f; t < n && !A->front_fork; t++) {
+            if (A->step_side[t]) continue;
+            if (std::find(A->step_waits[t].begin(), A->step_waits[t].end(), k) != A->step_waits[t].end() ||
+                A->steps[t].kind == ST_CYCLE_END)
+                break;
+            A->front_fork = true;
         }
     }
+    auto on_side = [&](size_t t) { return A->step_side[t] && A->front_fork; };
+    // A stream runs in order, so of several steps of one stream only the last
+    // is waited for, and none that an earlier wait of the same stream covers.
+    // (Regrowth records its event only when it fires, so it covers nothing.)
+    const StepAccess in = intake_access(A->plan);
+    auto prev_of = [&](const StepAccess& a, long& seen_main, long& seen_side, std::vector<size_t>& out) {
+        long m = -1, sd = -1;
+        for (size_t t = f; t < n; t++) {
+            if (A->steps[t].kind == ST_CYCLE_END || !conflict(acc[t], a)) continue;
+            if (A->steps[t].kind == ST_REGROW) out.push_back(t);
+            else (on_side(t) ? sd : m) = (long)t;
+        }
+        if (m > seen_main) out.push_back((size_t)(seen_main = m));
+        if (sd > seen_side) out.push_back((size_t)(seen_side = sd));
+        for (size_t t : out)
+            if (!on_side(t)) A->main_ev_needed[t] = 1;
+    };
+    long seen_main = -1, seen_side = -1;
+    for (size_t k = 0; k < f; k++) prev_of(acc[k], seen_main, seen_side, A->front_prev[k]);
+    seen_main = seen_side = -1;   // not every cycle has an intake before its front steps
+    prev_of(in, seen_main, seen_side, A->intake_prev);
+    long seen[2] = {-1, -1};      // latest front step that the main [0] and side [1] stream have waited for
+    bool intake_seen[2] = {};
+    A->front_join = true;
+    A->intake_ev_needed = false;
+    for (size_t t = f; t < n; t++) {
+        const int s = on_side(t) ? 1 : 0;
+        long j = -1;
+        for (size_t k = 0; k < f; k++)
+            if (conflict(acc[k], acc[t])) j = (long)k;
+        if (j > seen[s]) {
+            A->front_waits[t].push_back((size_t)j);
+            A->front_ev_needed[j] = 1;
+            seen[s] = j;
+            // Regrowth and the cycle's end do not launch on every cycle.
+            if (s == 0 && j == (long)f - 1 && t < A->n_body) A->front_join = false;
+            intake_seen[s] = true;   // the intake runs ahead of the front steps, on their stream
+        }
+        if (A->steps[t].kind != ST_CYCLE_END && conflict(in, acc[t]) && !intake_seen[s]) {
+            A->intake_readers[t] = 1;
+            A->intake_ev_needed = intake_seen[s] = true;
+        }
+    }
+    if (A->front_join) A->front_ev_needed[f - 1] = 1;
     cudaError_t e = cudaSuccess;
     if (!A->front) e = stream_like(A->stream(), &A->front);
     if (e == cudaSuccess && !A->intake_ev) e = cudaEventCreateWithFlags(&A->intake_ev, cudaEventDisableTiming);
@@ -647,14 +690,16 @@ int bm::schedule_area(bm_area_s* A) {
     // step of the cycle reads the cycle number after it advances). The side
     // stream runs its steps in order, so a main step's wait for side step j
     // joins every side step up to j.
-    A->end_in_tail = false;
-    if (n >= 2 && A->steps[n - 1].kind == ST_CYCLE_END && A->steps[n - 2].kind == ST_PYR_TAIL && !A->step_side[n - 2]) {
-        size_t joined = 0;   // side steps below this index have joined
-        for (size_t k = 0; k + 1 < n; k++)
-            if (!A->step_side[k])
-                for (size_t j : A->step_waits[k]) joined = std::max(joined, j + 1);
-        A->end_in_tail = A->last_side == SIZE_MAX || A->last_side < joined;
-    }
+    // With regrowth between them it folds on the cycles that do not regrow.
+    size_t m = n;   // the program up to regrowth and the cycle's end
+    while (m > 0 && (A->steps[m - 1].kind == ST_CYCLE_END || A->steps[m - 1].kind == ST_REGROW)) m--;
+    size_t joined = 0;   // side steps below this index have joined
+    for (size_t k = 0; k < m; k++)
+        if (!A->step_side[k])
+            for (size_t j : A->step_waits[k]) joined = std::max(joined, j + 1);
+    A->side_joined = A->last_side == SIZE_MAX || A->last_side < joined;
+    A->n_body = m;
+    A->end_in_tail = m > 0 && A->steps[m - 1].kind == ST_PYR_TAIL && !A->step_side[m - 1] && A->side_joined;
     for (cudaEvent_t ev : A->side_ev)
         if (ev) cudaEventDestroy(ev);
     A->side_ev.clear();
@@ -703,7 +748,7 @@ namespace {
 // Makes stream s wait for step t's event of the latest cycle that recorded it
 // (a side step's, or a main step's the front stream depends on).
 void wait_step(bm_area_s* A, size_t t, cudaStream_t s) {
-    if (A->last_side != SIZE_MAX && A->step_side[t]) cudaStreamWaitEvent(s, A->side_ev[t], 0);
+    if (A->step_side[t] && A->front_fork) cudaStreamWaitEvent(s, A->side_ev[t], 0);
     else if (t < A->main_ev.size() && A->main_ev[t]) cudaStreamWaitEvent(s, A->main_ev[t], 0);
 }
 
@@ -713,7 +758,9 @@ void wait_step(bm_area_s* A, size_t t, cudaStream_t s) {
 // the events the front stream's waits refer to).
 void front_begin(bm_area_s* A) {
     if (!A->front_last) A->mark_main();
+    if (A->front_mark == A->mark_seq) return;   // waited for already
     cudaStreamWaitEvent(A->front, A->main_mark, 0);
+    A->front_mark = A->mark_seq;
 }
 
 // The stream a frame intake goes to, with its waits on the previous cycle
@@ -728,7 +775,7 @@ cudaStream_t intake_begin(bm_area_s* A) {
 // After an intake's copies: later steps reading the inputs follow it, and with
 // `join` the main stream does too (an intake outside a cycling call).
 void intake_end(bm_area_s* A, cudaStream_t s, bool join) {
-    if (s != A->front) return;
+    if (s != A->front || !(join || A->intake_ev_needed)) return;
     cudaEventRecord(A->intake_ev, s);
     if (join) cudaStreamWaitEvent(A->stream(), A->intake_ev, 0);
 }
@@ -746,23 +793,24 @@ int enqueue_cycle(bm_area_s* A) {
     size_t last_side = SIZE_MAX;
     for (size_t k = nf; k < A->steps.size() && !A->profiling; k++)
         if (A->step_side[k]) last_side = k;
-    const bool fork = last_side != SIZE_MAX;
+    const bool fork = last_side != SIZE_MAX && (!front || A->front_fork);
     if (front) {
         front_begin(A);
         for (size_t k = 0; k < nf; k++) {
             for (size_t t : A->front_prev[k]) wait_step(A, t, A->front);
             exec_step(A, A->steps[k], A->front, false);
-            cudaEventRecord(A->front_ev[k], A->front);
+            if (A->front_ev_needed[k]) cudaEventRecord(A->front_ev[k], A->front);
         }
     }
     if (fork) {
         cudaEventRecord(A->ev_fork, main);
         cudaStreamWaitEvent(A->side, A->ev_fork, 0);
     }
-    // With end_in_tail the last pyramidal tail ends the cycle itself and the
-    // cycle-end step (the last) launches nothing.
-    const size_t n = A->steps.size() - (A->end_in_tail ? 1 : 0);
-    const bool regrow_fires = A->host_cycle % kRegrowPeriod == kRegrowPeriod - 1;
+    // With end_in_tail the last pyramidal tail ends the cycle itself, unless
+    // regrowth comes between.
+    const bool regrow_fires = A->regrow_blocks && A->host_cycle % kRegrowPeriod == kRegrowPeriod - 1;
+    const bool tail_ends = A->end_in_tail && !regrow_fires;
+    const size_t n = tail_ends ? A->n_body : A->steps.size();
     for (size_t k = nf; k < n; k++) {
         const bool on_side = fork && A->step_side[k];
         cudaStream_t s = on_side ? A->side : main;
@@ -773,13 +821,13 @@ int enqueue_cycle(bm_area_s* A) {
             for (size_t j : A->front_waits[k]) cudaStreamWaitEvent(s, A->front_ev[j], 0);
             if (A->intake_readers[k]) cudaStreamWaitEvent(s, A->intake_ev, 0);
         }
-        exec_step(A, A->steps[k], s, A->end_in_tail && k + 1 == n);
+        exec_step(A, A->steps[k], s, tail_ends && k + 1 == n);
         if (on_side) cudaEventRecord(A->side_ev[k], A->side);
         else if (front && A->main_ev_needed[k] && (A->steps[k].kind != ST_REGROW || regrow_fires))
             cudaEventRecord(A->main_ev[k], main);
     }
-    if (fork) cudaStreamWaitEvent(main, A->side_ev[last_side], 0);
-    if (front) cudaStreamWaitEvent(main, A->front_ev[nf - 1], 0);
+    if (fork && !A->side_joined) cudaStreamWaitEvent(main, A->side_ev[last_side], 0);
+    if (front && A->front_join) cudaStreamWaitEvent(main, A->front_ev[nf - 1], 0);
     A->front_last = front;
     A->host_cycle++;
     return A->samplers.empty() ? BM_OK : sample_after_cycle(A, main);

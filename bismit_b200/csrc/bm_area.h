@@ -173,7 +173,8 @@ struct bm_area_s {
     double prof_ms[bm::K_COUNT] = {};
     uint32_t launches = 0;   // kernel launches of the last enqueued cycle
     std::vector<Step> steps; // the cycle's stage program
-    bool end_in_tail = false;  // the last pyramidal tail also ends the cycle (no cycle-end launch)
+    bool end_in_tail = false;  // the last pyramidal tail also ends the cycle (no cycle-end launch) unless regrowth fires
+    size_t n_body = 0;         // steps before regrowth and the cycle's end
     // Two-stream form of the program (schedule_area): steps on the side
     // stream, the side steps each main step waits for, events and the stream.
     std::vector<uint8_t> step_side;
@@ -194,6 +195,12 @@ struct bm_area_s {
     std::vector<size_t> intake_prev;                     // steps of the previous cycle the intake waits for
     std::vector<uint8_t> intake_readers;                 // later steps reading what the intake writes
     std::vector<uint8_t> main_ev_needed;                 // main steps a front step or the intake waits for
+    std::vector<uint8_t> front_ev_needed;                // front steps a later step or the cycle's end waits for
+    bool front_fork = false;       // side steps keep their stream beside the front stream
+    bool front_join = true;        // the main stream has not joined the front stream by the cycle's last step
+    bool intake_ev_needed = false; // some later step waits for the intake itself
+    bool side_joined = true;       // the main stream has joined the side stream by the cycle's last step
+    uint64_t mark_seq = 0, front_mark = 0;   // records of main_mark, and the last one the front stream waited for
     std::bitset<BM_MAX_SLICES> front_ax_w;               // axon slices the front steps write
     std::vector<cudaEvent_t> front_ev, main_ev;
     cudaEvent_t intake_ev = nullptr;
@@ -244,7 +251,9 @@ struct bm_area_s {
     cudaStream_t intake_stream() const { return front_active() ? front : stream(); }
     // Marks the main stream's current position for the front stream.
     void mark_main() {
-        if (main_mark) cudaEventRecord(main_mark, stream());
+        if (!main_mark) return;
+        cudaEventRecord(main_mark, stream());
+        mark_seq++;
     }
     // Device error bits a completed cycle mirrored to the host (0: none seen).
     unsigned int seen_errors() const { return host_err ? *(volatile const unsigned int*)host_err : 0u; }
