@@ -119,7 +119,7 @@ struct FusedTuftArgs {
                                         // the footprint starts at 0
     uint32_t unit_l2;                   // log2 of the bytes of one unit (chunks_per_unit * 512)
     uint32_t stage_stride;              // bytes per ring buffer (synapse arrays + windows)
-    uint32_t win_bytes;                 // bytes per dendrite / cell-tuft window of a stage
+    uint32_t win_off, win_bytes;        // a stage's dendrite / cell-tuft windows: offset, bytes each
     uint32_t den_mis, cel_mis;          // how far the tuft's first dendrite and cell lie past a 16-byte boundary
     uint32_t geom;                      // specialised consumer for this shape (0: the general one)
     uint32_t fp_tma;                    // the footprint comes from a tensor box load (else consumers stage it)
@@ -581,20 +581,28 @@ __device__ __forceinline__ void build_footprint(const FusedTuftArgs& A, const Ti
     }
 }
 
-// Stage layout, per buffer of 4 x SB bytes of synapse arrays followed by the
-// windows: MODE 0 streams gidx (2 bytes a synapse) then strength, state and
-// (unless FCLEAN) flags; MODE 1 streams slc, v_ofs, u_ofs, strength, state,
-// flags. The common form (MODE 0, FCLEAN) takes SB synapses a stage; the wider
-// forms take SB / 2, so every form fits the same buffer. MODE 2 is MODE 0 for
-// tufts whose synapses start off a 16-byte boundary: arrays of SB + 16.
+// Stage layout: synapse arrays, then (at win_off) the windows. MODE 0: the
+// source data (offsets of 2 bytes a synapse, or codes of one and the slice
+// plane of a quarter), strength, state, (unless FCLEAN) flags. MODE 1: slc,
+// v_ofs, u_ofs, strength, state, flags. The common form (MODE 0, FCLEAN) takes
+// SB synapses a stage, the wider forms SB / 2, so every form fits the same
+// buffer of 4 x SB bytes. MODE 2 is MODE 0 for tufts whose synapses start off a
+// 16-byte boundary: arrays of SB + 16, and with 1024-synapse cells the source
+// data last, so that with codes a buffer takes 3.25 x SB and three CTAs fit an
+// SM (12 cycles of a 150 x 150 x 3 instance 1239 -> 1115 us; aligned cells, in
+// a batch of 24 instances, were 1 % slower that way).
 template <int MODE, bool FCLEAN>
 __device__ __forceinline__ uint32_t stage_syns(uint32_t SB) {
     return (MODE != 1 && FCLEAN) ? SB : SB / 2;
 }
 template <int MODE>
-__device__ __forceinline__ uint32_t arr_off(int which, uint32_t SB) {
+__device__ __forceinline__ bool src_last(const FusedTuftArgs& A) {
+    return MODE == 2 && A.stage_bytes > (uint32_t)kWarps * 512;
+}
+template <int MODE>
+__device__ __forceinline__ uint32_t arr_off(int which, uint32_t SX, bool last = false) {
     // which: 0 strength, 1 state, 2 flags
-    return MODE != 1 ? (2 + which) * SB : (3 + which) * SB;
+    return MODE != 1 ? (which + (last ? 0 : 2)) * SX : (3 + which) * SX;
 }
 
 // Consumer work of one stage: this warp's unit (a chunk, or a cell of
@@ -762,6 +770,8 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
     constexpr uint32_t SB = kWarps * UNIT;
     constexpr uint32_t SX = SB + (MIS ? 16 : 0);         // bytes of a 1-byte array in the stage
     constexpr uint32_t WIN = SB / 16 + 32;
+    constexpr bool LAST = MIS && HALVES == 2;            // src_last
+    constexpr uint32_t SRC = LAST ? 2 * SX : 0, STR = LAST ? 0 : 2 * SX, ST = STR + SX;
     constexpr uint32_t LPD = 1u << (SPD_L2 - 4);
     constexpr uint32_t LPC = 1u << LPC_L2;               // lanes a cell spans over its halves
     constexpr uint32_t LPCW = LPC > 32 ? 32u : LPC;      // lanes of a cell within one unit
@@ -772,7 +782,7 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
         C.old += HALVES * kCarryUnit;
         return;
     }
-    const uint8_t* wd = sb + 4 * SX;
+    const uint8_t* wd = sb + (LAST ? A.win_off : 4 * SX);
 #pragma unroll 1
     for (uint32_t h = 0; h < HALVES; h++, C.old += kCarryUnit) {
         const uint32_t so = (uint32_t)wib * UNIT + h * 512u + (uint32_t)lane * 16;
@@ -794,14 +804,14 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
         // Lanes past the tile's end gather from whatever the buffer held (any
         // 15-bit offset, and whatever codes decode to, is inside the CTA's
         // shared memory: kMinSmem, stray_reach) and drop the result.
-        const uint4 str4 = *(const uint4*)(sb + 2 * SX + so);
-        const uint4 st4 = *(const uint4*)(sb + 3 * SX + so);
+        const uint4 str4 = *(const uint4*)(sb + STR + so);
+        const uint4 st4 = *(const uint4*)(sb + ST + so);
         const uint32_t strw[4] = {str4.x, str4.y, str4.z, str4.w};
         const uint32_t stw[4] = {st4.x, st4.y, st4.z, st4.w};
         uint32_t gw[8];   // footprint offsets, two a word
         uint32_t edge_base = 0;
         if (A.compact) {
-            const uint4 c4 = *(const uint4*)(sb + so);
+            const uint4 c4 = *(const uint4*)(sb + SRC + so);
             const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w};
             const uint32_t base1 = code_base(A, G, min(off, G.syn_end - 16u) >> S_L2), base = base1 * 0x10001u;
             if (MIS) edge_base = base1;
@@ -812,13 +822,13 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
                 gw[w] = (x & 0x00F000F0u) * A.code_mul + (x + base);
             }
             if (A.compact == 2) {
-                const uint32_t sl = *(const uint32_t*)(sb + SX + so / 4);
+                const uint32_t sl = *(const uint32_t*)(sb + SRC + SX + so / 4);
 #pragma unroll
                 for (int w = 0; w < 8; w++) gw[w] += ((sl >> (2 * w)) & 0x00030003u) * A.fsz;
             }
         } else {
-            const uint4 g0 = *(const uint4*)(sb + 2 * so);
-            const uint4 g1 = *(const uint4*)(sb + 2 * so + 16);
+            const uint4 g0 = *(const uint4*)(sb + SRC + 2 * so);
+            const uint4 g1 = *(const uint4*)(sb + SRC + 2 * so + 16);
             const uint32_t ow[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
 #pragma unroll
             for (int w = 0; w < 8; w++) gw[w] = ow[w] & 0x7FFF7FFFu;
@@ -854,18 +864,18 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
                 const uint32_t e = u0 + (head ? n_on * 16 : 0u) + (uint32_t)lane;
                 uint32_t o;
                 if (A.compact) {
-                    const uint32_t c = sb[e];
+                    const uint32_t c = sb[SRC + e];
                     o = edge_base + (c >> 4) * A.fw + (c & 15u);
                     if (A.compact == 2)
-                        o += ((*(const uint32_t*)(sb + SX + (e & ~15u) / 4) >> slice_shift(e & 15u)) & 3u) * A.fsz;
+                        o += ((*(const uint32_t*)(sb + SRC + SX + (e & ~15u) / 4) >> slice_shift(e & 15u)) & 3u) * A.fsz;
                 } else {
-                    o = *(const uint16_t*)(sb + 2 * e) & 0x7FFFu;
+                    o = *(const uint16_t*)(sb + SRC + 2 * e) & 0x7FFFu;
                 }
                 const uint32_t a = halo[o];
                 const uint32_t i = pos + e - A.mis;
                 A.st[i] = (uint8_t)a;
-                A.fl[i] = sb[3 * SX + e] ? kSynPrevActiveFlag : (uint8_t)0;
-                if (head) edge = (a << 16) | ((int8_t)sb[2 * SX + e] >= 0 ? a : 0u);
+                A.fl[i] = sb[ST + e] ? kSynPrevActiveFlag : (uint8_t)0;
+                if (head) edge = (a << 16) | ((int8_t)sb[STR + e] >= 0 ? a : 0u);
             }
             const uint32_t lo = (raw_lo << 16) | sum_lo;
             const uint32_t past = __reduce_add_sync(0xFFFFFFFFu, edge), next = __shfl_down_sync(0xFFFFFFFFu, lo, 1);
@@ -962,6 +972,7 @@ __device__ __forceinline__ bool produce_tile(const FusedTuftArgs& A, const TileG
                                              volatile int& s_abort) {
     const uint32_t SB = stage_syns<MODE, FCLEAN>(A.stage_bytes);
     const uint32_t buf_bytes = A.stage_stride;
+    const bool last = src_last<MODE>(A);
     const uint32_t nst = A.nst;
     for (uint32_t pos = G.syn0; pos < G.syn_end; pos += SB) {
         if (s_abort) return false;
@@ -995,7 +1006,7 @@ __device__ __forceinline__ bool produce_tile(const FusedTuftArgs& A, const TileG
         const uint32_t cb = ((A.cel_mis + ((pos + nb) >> A.S_l2) + 15) & ~15u) - c0;
         n_arr_bytes += db + (TUFT ? 4 * cb : 0u);
         mbar_arrive_expect_tx(&full[pb], n_arr_bytes);
-        uint8_t* wd = dst + 4 * (A.stage_bytes + (MODE == 2 ? 16 : 0));
+        uint8_t* wd = dst + (MODE == 2 ? A.win_off : 4 * A.stage_bytes);
         bulk_g2s(wd, A.den_act - A.den_mis + d0, db, &full[pb]);
         if (TUFT) {
             bulk_g2s(wd + A.win_bytes, A.t_bid - A.cel_mis + c0, cb, &full[pb]);
@@ -1003,20 +1014,22 @@ __device__ __forceinline__ bool produce_tile(const FusedTuftArgs& A, const TileG
             bulk_g2s(wd + 3 * A.win_bytes, A.t_bst - A.cel_mis + c0, cb, &full[pb]);
             bulk_g2s(wd + 4 * A.win_bytes, A.t_st - A.cel_mis + c0, cb, &full[pb]);
         }
+        const uint32_t src = last ? 2 * SX : 0u;
         if (MODE != 1 && A.compact) {
-            bulk_g2s(dst, (const uint8_t*)A.gidx + pos, nw, &full[pb]);
-            if (A.compact == 2) bulk_g2s(dst + SX, A.gslc + pos / 4, plane, &full[pb]);
+            bulk_g2s(dst + src, (const uint8_t*)A.gidx + pos, nw, &full[pb]);
+            if (A.compact == 2)
+                bulk_g2s(dst + src + SX, A.gslc + pos / 4, plane, &full[pb]);
         } else if (MODE != 1) {
-            bulk_g2s(dst, A.gidx + pos, 2 * nw, &full[pb]);
+            bulk_g2s(dst + src, A.gidx + pos, 2 * nw, &full[pb]);
         } else {
             bulk_g2s(dst, A.slc + pos, nb, &full[pb]);
             bulk_g2s(dst + SB, A.vofs + pos, nb, &full[pb]);
             bulk_g2s(dst + 2 * SB, A.uofs + pos, nb, &full[pb]);
         }
         const uint32_t mis = MODE == 2 ? A.mis : 0u;
-        bulk_g2s(dst + arr_off<MODE>(0, SX), A.str - mis + pos, nw, &full[pb]);
-        bulk_g2s(dst + arr_off<MODE>(1, SX), A.st - mis + pos, nw, &full[pb]);
-        if (!FCLEAN) bulk_g2s(dst + arr_off<MODE>(2, SB), A.fl + pos, nb, &full[pb]);
+        bulk_g2s(dst + arr_off<MODE>(0, SX, last), A.str - mis + pos, nw, &full[pb]);
+        bulk_g2s(dst + arr_off<MODE>(1, SX, last), A.st - mis + pos, nw, &full[pb]);
+        if (!FCLEAN) bulk_g2s(dst + arr_off<MODE>(2, SB, last), A.fl + pos, nb, &full[pb]);
         if (++pb == nst) { pb = 0; ps.pround++; }
     }
     return true;
@@ -1616,7 +1629,10 @@ void plan_tuft_form(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t
     // Windows: up to SB / 16 dendrites (or cells) per stage, widened by up to
     // 15 at both ends.
     const uint32_t win_bytes = SB / 16 + 32;
-    const uint32_t buf_bytes = 4 * (SB + (FT.mis ? 16 : 0)) + 5 * win_bytes;
+    if (!fast_shape(S, spd, L.kind == BM_LYR_PYRAMIDAL)) compact = 0;
+    const uint32_t SX = SB + (FT.mis ? 16 : 0);
+    FT.win_off = compact && FT.mis && cpu == 2 ? 3 * SX + SB / 4 + 16 : 4 * SX;
+    const uint32_t buf_bytes = FT.win_off + 5 * win_bytes;
     // The footprint sits at the start of dynamic shared memory (gathers then
     // address it with a constant base), the ring after it.
     const uint64_t ring_off = std::max<uint64_t>(((halo + 127) / 128) * 128, FT.mis ? kSegBytes : 0);
@@ -1637,7 +1653,7 @@ void plan_tuft_form(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t
     FT.stage_bytes = SB;
     FT.stage_stride = buf_bytes;
     FT.win_bytes = win_bytes;
-    FT.compact = consumer_shape(FT, S, spd, L.kind == BM_LYR_PYRAMIDAL) ? compact : 0u;
+    FT.compact = compact;
     FT.ring_off = (uint32_t)ring_off;
     FT.smem = (uint32_t)smem;
     FT.src_vs = vs;
@@ -1950,6 +1966,7 @@ void make_args(FusedTuftArgs& A, const FusedArea& F, const uint8_t* axns, const 
         A.ring_off = FT.ring_off;
         A.unit_l2 = 9 + ilog2(A.chunks_per_unit);
         A.stage_stride = FT.stage_stride;
+        A.win_off = FT.win_off;
         A.win_bytes = FT.win_bytes;
         A.den_mis = (uint32_t)(T.den_idz & 15);
         A.cel_mis = (uint32_t)(T.cel_idz & 15);
@@ -2009,25 +2026,25 @@ int prepare_fused_batch(FusedBatch& B, const std::vector<FusedJob>& jobs, const 
         if (!FT.ok || !FT.tiled || !FT.gidx || (J.L->kind == BM_LYR_PYRAMIDAL) != tuft) return BM_OK;
         sms = (uint32_t)J.F->sms;
     }
-    // Jobs of one stage geometry share launches (a launch's ring is uniform,
-    // and jobs with smaller stages then keep three CTAs per SM). Unaligned
-    // tufts' stages are a little larger: they get launches of their own.
-    std::vector<uint32_t> strides;
+    // Jobs of one stage size share launches (a launch's ring is uniform, its
+    // buffers its largest job's, and jobs with smaller stages then keep three
+    // CTAs per SM); unaligned tufts, whose kernel is another, get their own.
+    std::vector<std::pair<uint32_t, bool>> classes;
     for (const FusedJob& J : jobs) {
-        const uint32_t st = J.F->t[J.layer][J.t].stage_stride;
-        if (std::find(strides.begin(), strides.end(), st) == strides.end()) strides.push_back(st);
+        const FusedTuft& FT = J.F->t[J.layer][J.t];
+        const std::pair<uint32_t, bool> c{FT.stage_bytes, FT.mis != 0};
+        if (std::find(classes.begin(), classes.end(), c) == classes.end()) classes.push_back(c);
     }
-    std::sort(strides.begin(), strides.end());
-    for (uint32_t stride : strides) {
+    std::sort(classes.begin(), classes.end());
+    for (const auto& [stage_bytes, mis] : classes) {
         std::vector<const FusedJob*> cls;
-        bool mis = false;
-        uint32_t halo = 0;
+        uint32_t halo = 0, stride = 0;
         uint64_t reach = kMinSmem;
         for (const FusedJob& J : jobs) {
             const FusedTuft& FT = J.F->t[J.layer][J.t];
-            if (FT.stage_stride != stride) continue;
+            if (FT.stage_bytes != stage_bytes || (FT.mis != 0) != mis) continue;
             cls.push_back(&J);
-            mis = FT.mis != 0;
+            stride = std::max(stride, FT.stage_stride);
             halo = std::max(halo, ((FT.nrec * FT.fsz + 127) / 128) * 128);
             reach = std::max(reach, stray_reach(FT.fsz, FT.fw));
         }

@@ -29,7 +29,7 @@ struct FusedTuft {
     uint32_t stage_bytes = 0;
     uint32_t ring_off = 0;   // ring offset in dynamic shared memory (the footprint is at 0)
     uint32_t stage_stride = 0;   // bytes per ring buffer
-    uint32_t win_bytes = 0;      // bytes per dendrite / cell-tuft window
+    uint32_t win_off = 0, win_bytes = 0;   // a stage's dendrite / cell-tuft windows: offset, bytes each
     uint32_t src_vs = 0, src_us = 0, src_vsz = 0, src_usz = 0;
     uint32_t src_idz[8] = {};
     uint32_t tile_target = 0;    // synapses per tile asked for (0: chosen from the tuft's size)
