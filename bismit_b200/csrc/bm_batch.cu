@@ -75,25 +75,22 @@ struct BatchCtl {
 // An unfused tuft's stages: by 16- or 4-byte windows (bm_seg.cuh), or a thread
 // per cell (tuft_cell_item; tufts of a few synapses).
 constexpr int BK_TUFT_SEG16 = 100, BK_TUFT_SEG4 = 101, BK_TUFT_CELLS = 102;
+// Pyramidal tails with folded tufts (TailFold).
+constexpr int BK_TAIL_ONE = 103, BK_TAIL_ANY = 104;
 
 constexpr uint32_t kCellBlock = 128;
 constexpr uint32_t kIntakeBlock = 256;
 constexpr uint32_t kIntakePerThread = 4;
 
+// The job of this block: the last that starts at or before it. Every thread
+// looks at one job, so a table costs one trip to memory (a binary search by one
+// thread cost one a step).
 template <class J>
 __device__ __forceinline__ uint32_t block_job(const J* __restrict__ jobs, uint32_t n_jobs) {
-    __shared__ uint32_t s_j;
-    if (threadIdx.x == 0) {
-        uint32_t lo = 0, hi = n_jobs;
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (jobs[mid].block0 <= blockIdx.x) lo = mid;
-            else hi = mid;
-        }
-        s_j = lo;
-    }
-    __syncthreads();
-    return s_j;
+    uint32_t n = 0;
+    for (uint32_t k = 0; k < n_jobs; k += blockDim.x)
+        n += (uint32_t)__syncthreads_count(k + threadIdx.x < n_jobs && jobs[k + threadIdx.x].block0 <= blockIdx.x);
+    return n - 1;
 }
 
 template <int ST>
@@ -108,10 +105,6 @@ __global__ void __launch_bounds__(kCellBlock)
                        rnd_at(J.L.rnd_key_ssc_mtp, J.ctl->cycle), J.learn != 0, i, i < J.n);
         return;
     }
-    if (ST == ST_PYR_TAIL) {
-        pyr_tail_warp(J.axns, J.slices, J.L, J.ctrl, J.learn != 0, J.ctl, i, i < J.n, J.tufts);
-        return;
-    }
     if (i >= J.n) return;
     switch (ST) {
     case ST_SSC_CYCLE: ssc_cycle_item(J.L, i); break;
@@ -123,7 +116,7 @@ __global__ void __launch_bounds__(kCellBlock)
     case ST_DST_MTP: tft_dst_mtp_item(J.axns, J.L, J.x, rnd_at(J.L.tft[J.x].rnd_key_mtp, J.ctl->cycle), i); break;
     case ST_SSC_MTP: ssc_mtp_item(J.axns, J.L, rnd_at(J.L.rnd_key_ssc_mtp, J.ctl->cycle), i); break;
     case BK_TUFT_CELLS:
-        tuft_cell_item(J.axns, J.slices, J.L, J.x, rnd_at(J.L.tft[J.x].rnd_key_den, J.ctl->cycle), i);
+        tuft_cells_item(J.axns, J.slices, J.L, J.x, rnd_at(J.L.tft[J.x].rnd_key_den, J.ctl->cycle), i);
         break;
     default: break;
     }
@@ -172,11 +165,12 @@ __global__ void k_batch_begin(BatchCtl* bc, const uint8_t* frames, uint64_t fram
 // (64 registers, none spilled; 72 and seven blocks as an instantiation of
 // k_batch_cells): a batch's tail covers every area's cells in several waves,
 // and the extra block per SM took batch_64's tail from 0.120 to 0.084 ms.
-__global__ void __launch_bounds__(kCellBlock, 8) k_batch_tail(const CellJob* __restrict__ jobs, uint32_t n_jobs) {
+template <int FOLD>
+__global__ void __launch_bounds__(kCellBlock, FOLD == FOLD_NONE ? 8 : 4) k_batch_tail(const CellJob* __restrict__ jobs, uint32_t n_jobs) {
     pdl_begin();
     const CellJob& J = jobs[block_job(jobs, n_jobs)];
     const uint32_t i = (blockIdx.x - J.block0) * kCellBlock + threadIdx.x;
-    pyr_tail_warp(J.axns, J.slices, J.L, J.ctrl, J.learn != 0, J.ctl, i, i < J.n, J.tufts);
+    pyr_tail_warp<FOLD>(J.axns, J.slices, J.L, J.ctrl, J.learn != 0, J.ctl, i, i < J.n, J.tufts);
 }
 
 void launch_cells(int st, const CellJob* jobs, uint32_t n_jobs, uint32_t n_blocks, cudaStream_t s) {
@@ -193,7 +187,9 @@ void launch_cells(int st, const CellJob* jobs, uint32_t n_jobs, uint32_t n_block
         BM_CELLS(ST_DST_MTP)
         BM_CELLS(ST_SSC_MTP)
         BM_CELLS(ST_INHIB_MTP)
-    case ST_PYR_TAIL: launch_pdl(k_batch_tail, n_blocks, kCellBlock, 0, s, jobs, n_jobs); break;
+    case BK_TAIL_ONE: launch_pdl(k_batch_tail<FOLD_ONE>, n_blocks, kCellBlock, 0, s, jobs, n_jobs); break;
+    case BK_TAIL_ANY: launch_pdl(k_batch_tail<FOLD_ANY>, n_blocks, kCellBlock, 0, s, jobs, n_jobs); break;
+    case ST_PYR_TAIL: launch_pdl(k_batch_tail<FOLD_NONE>, n_blocks, kCellBlock, 0, s, jobs, n_jobs); break;
         BM_CELLS(BK_TUFT_CELLS)
     case BK_TUFT_SEG16: launch_pdl(k_batch_tuft_seg<16>, n_blocks, kSegBlock, 0, s, jobs, n_jobs); break;
     case BK_TUFT_SEG4: launch_pdl(k_batch_tuft_seg<4>, n_blocks, kSegBlock, 0, s, jobs, n_jobs); break;
@@ -397,6 +393,11 @@ int add_cells(bm_ctx ctx, bm_batch_s::StepPlan& p, int k) {
         jobs.push_back(J);
     }
     if (blocks > 0x7FFFFFFFull) return set_err(BM_ERR_UNSUPPORTED, "batched step of too many blocks");
+    if (k == ST_PYR_TAIL) {
+        TailFold f = FOLD_NONE;
+        for (const CellJob& J : jobs) f = std::max(f, tail_fold(J.L, J.tufts));
+        if (f != FOLD_NONE) k = f == FOLD_ONE ? BK_TAIL_ONE : BK_TAIL_ANY;
+    }
     bm_batch_s::CellLaunch c{k, nullptr, (uint32_t)jobs.size(), (uint32_t)blocks};
     cudaError_t e = dev_alloc(ctx, &c.d_jobs, jobs.size() * sizeof(CellJob));
     if (e == cudaSuccess)

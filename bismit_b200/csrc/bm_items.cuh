@@ -107,6 +107,8 @@ __device__ __forceinline__ uint8_t inhib_simple_cell(uint8_t* __restrict__ axns,
     bool safe;
     uint32_t axi = axn_idx(slices[s + L.base_slc], (uint32_t)v, 0, (uint32_t)u, 0, false, safe);
     uint8_t cel_state = safe ? cs[c] : (uint8_t)0;
+    uint8_t* act = L.buf[BM_BUF_CEL_ACTIVITIES];
+    const uint8_t act0 = act[c];   // ahead of the stores, so its latency overlaps the neighbours'
     int uninhibited = 1;
     int horizon = radius + kInhibHorizOffset;
     int infl_max = horizon * horizon;
@@ -126,8 +128,7 @@ __device__ __forceinline__ uint8_t inhib_simple_cell(uint8_t* __restrict__ axns,
     const uint8_t out = (uint8_t)(uninhibited * cel_state);
     axns[axi] = out;
     int axon_active = uninhibited & (cel_state != 0);
-    uint8_t* act = L.buf[BM_BUF_CEL_ACTIVITIES];
-    act[c] = update_activity(act[c], axon_active, rnd, (int32_t)((uint32_t)cel_state | c), kCellActivityDecay);
+    act[c] = update_activity(act0, axon_active, rnd, (int32_t)((uint32_t)cel_state | c), kCellActivityDecay);
     return out;
 }
 __device__ __forceinline__ uint8_t inhib_simple_item(uint8_t* __restrict__ axns, const SliceRec* __restrict__ slices,
@@ -266,6 +267,67 @@ __device__ __forceinline__ void tuft_cell_item(const uint8_t* __restrict__ axns,
     }
     for (uint32_t d = 0; d < T.dpt; d++) den_cycle_item(L, t, rnd_den, (uint64_t)c * T.dpt + d);
     if (L.kind == BM_LYR_PYRAMIDAL) tft_cycle_item(L, t, c);
+}
+
+// What the soma and learning steps read of a tuft.
+struct TuftOut {
+    uint8_t state, best_raw, prev_raw, prev_id;
+};
+
+// tuft_cell_item for a pyramidal tuft of one synapse a cell, every input loaded
+// before anything is stored: the loads of a cell then cost two trips to memory
+// (the source, then its axon) in place of one per stage. 28,800 cells, a thread
+// each: 4.7 us cold, 8.3 through tuft_cell_item; 826,000 of a batch 20.3, 38.5;
+// a 64 x 64 area's tail with the tuft folded in 7.7, 12.2.
+__device__ __forceinline__ TuftOut tuft_cell1_item(const uint8_t* __restrict__ axns,
+                                                   const SliceRec* __restrict__ slices, const DevLayer& L, uint32_t t,
+                                                   int32_t rnd, uint32_t c) {
+    const DevTuft& T = L.tft[t];
+    const uint64_t si = T.syn_idz + c, di = T.den_idz + c, ci = T.cel_idz + c;
+    const uint8_t slc = L.buf[BM_BUF_SYN_SRC_SLC_IDS][si];
+    const int vo = (int8_t)L.buf[BM_BUF_SYN_SRC_COL_V_OFFS][si], uo = (int8_t)L.buf[BM_BUF_SYN_SRC_COL_U_OFFS][si];
+    const int8_t str = (int8_t)L.buf[BM_BUF_SYN_STRENGTHS][si];
+    const uint8_t st0 = L.buf[BM_BUF_SYN_STATES][si], fl0 = L.buf[BM_BUF_SYN_FLAG_SETS][si];
+    const uint8_t act0 = L.buf[BM_BUF_DEN_ACTIVITIES][di];
+    const uint8_t bid = L.buf[BM_BUF_TFT_BEST_DEN_IDS][ci], braw = L.buf[BM_BUF_TFT_BEST_DEN_STATES_RAW][ci];
+    const uint8_t bst = L.buf[BM_BUF_TFT_BEST_DEN_STATES][ci], tst = L.buf[BM_BUF_TFT_STATES][ci];
+    SliceRec r = slices[T.src_slc];   // beside the source: most pools have one slice
+    const uint32_t cols = L.v_size * L.u_size, rem = c % cols;
+    if (slc != T.src_slc) r = slices[slc];
+    bool safe;
+    const uint32_t ai = axn_idx(r, rem / L.u_size, vo, rem % L.u_size, uo, false, safe);   // one synapse: the scalar form
+    const uint32_t st = syn_fire(safe ? axns[ai] : (uint8_t)0);
+    const uint32_t pos = str >= 0 ? st : 0u;
+    const int active = pos > T.thresh;
+    const uint32_t seed = (st + T.thresh) | (uint32_t)di;
+    const uint32_t d_raw = min(st >> 4, 255u), d_st = active ? min(pos >> 4, 255u) : 0u;
+    const bool is_max = d_st >= (1u << (T.mad_l2 + 8));
+    const uint8_t ts = is_max ? (uint8_t)255 : (uint8_t)(d_st >> T.mad_l2);
+    L.buf[BM_BUF_SYN_FLAG_SETS][si] = (uint8_t)((fl0 & ~kSynPrevActiveFlag) | (st0 ? kSynPrevActiveFlag : 0));
+    L.buf[BM_BUF_SYN_STATES][si] = (uint8_t)st;
+    L.buf[BM_BUF_DEN_ACTIVITIES][di] = update_activity(act0, active, rnd, (int32_t)seed, kDendriteActivityDecay);
+    L.buf[BM_BUF_DEN_STATES_RAW][di] = (uint8_t)d_raw;
+    L.buf[BM_BUF_DEN_STATES][di] = (uint8_t)d_st;
+    L.buf[BM_BUF_TFT_PREV_BEST_DEN_IDS][ci] = bid;
+    L.buf[BM_BUF_TFT_PREV_BEST_DEN_STATES_RAW][ci] = braw;
+    L.buf[BM_BUF_TFT_PREV_BEST_DEN_STATES][ci] = bst;
+    L.buf[BM_BUF_TFT_PREV_STATES][ci] = tst;
+    L.buf[BM_BUF_TFT_BEST_DEN_IDS][ci] = 0;
+    L.buf[BM_BUF_TFT_BEST_DEN_STATES_RAW][ci] = (uint8_t)d_raw;
+    L.buf[BM_BUF_TFT_BEST_DEN_STATES][ci] = (uint8_t)d_st;
+    L.buf[BM_BUF_TFT_STATES][ci] = ts;
+    return {ts, (uint8_t)d_raw, braw, bid};
+}
+
+// A pyramidal tuft of a few synapses a cell, for cell c.
+__device__ __forceinline__ TuftOut tuft_cells_item(const uint8_t* __restrict__ axns,
+                                                   const SliceRec* __restrict__ slices, const DevLayer& L, uint32_t t,
+                                                   int32_t rnd, uint32_t c) {
+    if (L.tft[t].spt == 1) return tuft_cell1_item(axns, slices, L, t, rnd, c);
+    tuft_cell_item(axns, slices, L, t, rnd, c);
+    const uint64_t ci = L.tft[t].cel_idz + c;
+    return {L.buf[BM_BUF_TFT_STATES][ci], L.buf[BM_BUF_TFT_BEST_DEN_STATES_RAW][ci],
+            L.buf[BM_BUF_TFT_PREV_BEST_DEN_STATES_RAW][ci], L.buf[BM_BUF_TFT_PREV_BEST_DEN_IDS][ci]};
 }
 
 // The strength updates of learning, for every learning cell of the warp
@@ -456,11 +518,23 @@ __host__ __device__ __forceinline__ uint64_t tail_items(uint32_t depth, uint32_t
     return (uint64_t)cols * g;
 }
 
+// Tufts folded into a tail: none, all of one synapse a cell, or any. A template
+// parameter: the general form's registers would make the others spill.
+enum TailFold { FOLD_NONE, FOLD_ONE, FOLD_ANY };
+inline TailFold tail_fold(const DevLayer& L, uint32_t tufts) {
+    TailFold f = FOLD_NONE;
+    for (uint32_t t = 0; t < L.n_tufts; t++)
+        if ((tufts >> t) & 1u) f = L.tft[t].spt == 1 && f != FOLD_ANY ? FOLD_ONE : FOLD_ANY;
+    return f;
+}
+
 // Item t of the tail: lane d of column t / G, G = tail_group(depth), or the
 // whole column t when the column is deeper than kTailDepth.
+template <int FOLD>
 __device__ __forceinline__ void pyr_tail_warp(uint8_t* __restrict__ axns, const SliceRec* __restrict__ slices,
                                               const DevLayer& L, int ctrl, bool learn, const AreaCtl* ctl,
-                                              uint32_t item, bool valid_item, uint32_t tufts = 0) {
+                                              uint32_t item, bool valid_item, uint32_t tufts) {
+    if (FOLD == FOLD_NONE) tufts = 0;
     const uint32_t cols = L.v_size * L.u_size;
     const int lane = threadIdx.x & 31;
     uint8_t* cfl = L.buf[BM_BUF_CEL_FLAG_SETS];
@@ -469,29 +543,42 @@ __device__ __forceinline__ void pyr_tail_warp(uint8_t* __restrict__ axns, const 
         const uint32_t col = item / G, d = item & (G - 1);
         const bool valid = valid_item && col < cols && d < L.depth;
         const uint32_t c = d * cols + col;
-        // Tufts the fused tuft kernel does not take, folded in: their four
-        // stages for this cell, which the soma reads next.
-        for (uint32_t t = 0; tufts && t < L.n_tufts; t++)
-            if (((tufts >> t) & 1) && valid) tuft_cell_item(axns, slices, L, t, rnd_at(L.tft[t].rnd_key_den, ctl->cycle), c);
         const bool prx_on = (L.enabled_flags & kDenBasalProximalFlag) != 0;
         const bool dst_on = (L.enabled_flags & kDenBasalDistalFlag) != 0;
         uint8_t prx = 0, dst = 0, f = 0, ax = 0;
-        uint8_t praw[BM_MAX_TUFTS] = {}, pid[BM_MAX_TUFTS] = {};   // distal tufts' previous best
+        // Distal tufts' previous best raw states and ids, a byte a tuft.
+        static_assert(BM_MAX_TUFTS <= 4, "a byte a tuft in a word");
+        uint32_t praw = 0, pid = 0;
+        auto folded = [&](uint32_t t) { return ((tufts >> t) & 1u) != 0; };
         if (valid) {
-            prx = prx_on ? L.buf[BM_BUF_TFT_STATES][(uint64_t)L.prx_id * L.cells + c] : (uint8_t)0;
-            dst = dst_on ? L.buf[BM_BUF_TFT_BEST_DEN_STATES_RAW][(uint64_t)L.dst_id * L.cells + c] : (uint8_t)0;
+            // What no folded tuft writes, ahead of them.
+            if (prx_on && !folded(L.prx_id)) prx = L.buf[BM_BUF_TFT_STATES][(uint64_t)L.prx_id * L.cells + c];
+            if (dst_on && !folded(L.dst_id)) dst = L.buf[BM_BUF_TFT_BEST_DEN_STATES_RAW][(uint64_t)L.dst_id * L.cells + c];
             if (learn) {
                 f = cfl[c];
 #pragma unroll
                 for (uint32_t t = 0; t < BM_MAX_TUFTS; t++) {
-                    if (t < L.n_tufts && L.tft[t].den_kind == BM_DEN_DISTAL) {
+                    if (t < L.n_tufts && L.tft[t].den_kind == BM_DEN_DISTAL && !folded(t)) {
                         const uint32_t tci = c + (uint32_t)L.tft[t].cel_idz;
-                        praw[t] = L.buf[BM_BUF_TFT_PREV_BEST_DEN_STATES_RAW][tci];
-                        pid[t] = L.buf[BM_BUF_TFT_PREV_BEST_DEN_IDS][tci];
+                        praw |= (uint32_t)L.buf[BM_BUF_TFT_PREV_BEST_DEN_STATES_RAW][tci] << (8 * t);
+                        pid |= (uint32_t)L.buf[BM_BUF_TFT_PREV_BEST_DEN_IDS][tci] << (8 * t);
                     }
                 }
             }
             if (ctrl == 0) ax = axns[L.axn_idz + c];
+            // Tufts of a few synapses, folded in: their four stages for this
+            // cell, which the soma reads next.
+#pragma unroll 1
+            for (uint32_t t = 0; tufts && t < L.n_tufts; t++) {
+                if (!folded(t)) continue;
+                const int32_t rnd = rnd_at(L.tft[t].rnd_key_den, ctl->cycle);
+                const TuftOut o = FOLD == FOLD_ONE ? tuft_cell1_item(axns, slices, L, t, rnd, c)
+                                                   : tuft_cells_item(axns, slices, L, t, rnd, c);
+                if (t == L.prx_id && prx_on) prx = o.state;
+                if (t == L.dst_id && dst_on) dst = o.best_raw;
+                praw |= (uint32_t)o.prev_raw << (8 * t);
+                pid |= (uint32_t)o.prev_id << (8 * t);
+            }
         }
         // pyr_cycle, cl/bismit.cl:961-1022 (as pyr_cycle_item).
         const int p_active = prx != 0;
@@ -520,7 +607,7 @@ __device__ __forceinline__ void pyr_tail_warp(uint8_t* __restrict__ axns, const 
             if (T.den_kind != BM_DEN_DISTAL) continue;
             const int32_t rnd = rnd_at(T.rnd_key_mtp, ctl->cycle);
             uint32_t z, n;
-            dst_mtp_range_of(L, T, c, f, ax != 0, valid, praw[t], pid[t], z, n);
+            dst_mtp_range_of(L, T, c, f, ax != 0, valid, (uint8_t)(praw >> (8 * t)), (uint8_t)(pid >> (8 * t)), z, n);
             learn_runs<false>(L, rnd, __ballot_sync(0xFFFFFFFFu, n != 0), z, T.spd, lane);
             f = (uint8_t)((f & ~kCelPrevActiveFlag) | (ax ? kCelPrevActiveFlag : 0));
         }

@@ -113,7 +113,7 @@ __global__ void k_tuft_cells(const uint8_t* __restrict__ axns, const SliceRec* _
                              uint32_t t, const AreaCtl* ctl) {
     pdl_begin();
     uint32_t c = (uint32_t)gtid();
-    if (c < L.cells) tuft_cell_item(axns, slices, L, t, rnd_at(L.tft[t].rnd_key_den, ctl->cycle), c);
+    if (c < L.cells) tuft_cells_item(axns, slices, L, t, rnd_at(L.tft[t].rnd_key_den, ctl->cycle), c);
 }
 
 // W: bytes of each thread's window (bm_seg.cuh). 16 while that still gives
@@ -146,13 +146,15 @@ __global__ void __launch_bounds__(128) k_inhib_mtp(uint8_t* __restrict__ axns, c
 // With end_cycle, the last block to finish also ends the cycle (the cycle-end
 // launch folded in): every block has read the cycle number by then. Twelve
 // blocks of 128 per SM (40 registers): area_256's 262,144 cells then need 1.15
-// waves of warps instead of the 1.54 that 54 registers allowed.
-__global__ void __launch_bounds__(128, 12) k_pyr_tail(uint8_t* __restrict__ axns, const SliceRec* __restrict__ slices,
-                                                  DevLayer L, int ctrl, int learn, AreaCtl* ctl, uint32_t tufts,
-                                                  int end) {
+// waves of warps instead of the 1.54 that 54 registers allowed. With folded
+// tufts there are few cells: six, and nothing spilled.
+template <int FOLD>
+__global__ void __launch_bounds__(128, FOLD == FOLD_NONE ? 12 : 6)
+    k_pyr_tail(uint8_t* __restrict__ axns, const SliceRec* __restrict__ slices, DevLayer L, int ctrl, int learn,
+               AreaCtl* ctl, uint32_t tufts, int end) {
     pdl_begin();
     const uint64_t i = gtid();
-    pyr_tail_warp(axns, slices, L, ctrl, learn != 0, ctl, (uint32_t)i, i < tail_items(L.depth, L.v_size * L.u_size),
+    pyr_tail_warp<FOLD>(axns, slices, L, ctrl, learn != 0, ctl, (uint32_t)i, i < tail_items(L.depth, L.v_size * L.u_size),
                   tufts);
     if (!end) return;
     __syncthreads();
@@ -374,7 +376,9 @@ void launch_inhib_mtp(uint8_t* axns, const SliceRec* slices, const DevLayer& L, 
 }
 void launch_pyr_tail(uint8_t* axns, const SliceRec* slices, const DevLayer& L, int ctrl, bool learn, AreaCtl* ctl,
                      cudaStream_t s, uint32_t tufts, bool end) {
-    launch_pdl(k_pyr_tail, nblk(tail_items(L.depth, L.v_size * L.u_size), 128), 128, 0, s, axns, slices, L, ctrl,
+    const TailFold f = tail_fold(L, tufts);
+    auto kern = f == FOLD_NONE ? k_pyr_tail<FOLD_NONE> : f == FOLD_ONE ? k_pyr_tail<FOLD_ONE> : k_pyr_tail<FOLD_ANY>;
+    launch_pdl(kern, nblk(tail_items(L.depth, L.v_size * L.u_size), 128), 128, 0, s, axns, slices, L, ctrl,
                learn ? 1 : 0, ctl, tufts, end ? 1 : 0);
 }
 void launch_tft_dst_mtp_plain(const uint8_t* axns, const DevLayer& L, uint32_t t, const AreaCtl* ctl,

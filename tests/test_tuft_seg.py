@@ -124,3 +124,60 @@ def test_unaligned_sources_moved(shape, batched):
         b.close()
     a.close()
     ctx.close()
+
+
+def _small(side, depth, pyr):
+    """configs.instance_area with the pyramidal cells given."""
+    lmaps, areas = M.LayerMapSchemeList(), M.AreaSchemeList()
+    ext = M.LayerMapScheme("v0_lm", M.LayerMapKind.Subcortical)
+    ext.layer(M.LayerScheme.define("ganglion").depth(1).axonal(M.AxonTopology.Spatial)
+              .axon_domain(M.AxonDomain.output([M.THAL_SP])))
+    lmaps.add(ext)
+    areas.area(M.AreaScheme("v0", "v0_lm", side))
+    lm = M.LayerMapScheme("visual", M.LayerMapKind.Cortical)
+    lm.layer(M.LayerScheme.define("aff_in").axonal(M.AxonTopology.Spatial)
+             .axon_domain(M.AxonDomain.input([(M.InputTrack.Afferent, [M.THAL_SP])])))
+    lm.layer(M.LayerScheme.define("iv").depth(1).tags(M.LayerTags.PSAL).axon_domain(M.AxonDomain.Local)
+             .cellular(M.CellScheme.spiny_stellate()
+                       .tft(M.TuftScheme.basal().proximal().syns_per_den(32)
+                            .src_lyr(M.TuftSourceLayer.define("aff_in").syn_reach(6).prevalence(1)))))
+    lm.layer(M.LayerScheme.define("iv_inhib").cellular(
+        M.CellScheme.control(M.ControlCellKind.InhibitoryBasketSurround("iv", 4), 0)))
+    lm.layer(M.LayerScheme.define("iii").depth(depth).tags(M.LayerTags.PTAL)
+             .axon_domain(M.AxonDomain.output([M.THAL_SP])).cellular(pyr))
+    lm.layer(M.LayerScheme.define("iii_col").cellular(
+        M.CellScheme.control(M.ControlCellKind.IntraColumnInhib("iii"), 0)))
+    lmaps.add(lm)
+    areas.area(M.AreaScheme("v1", "visual", side).eff_areas(["v0"]))
+    return lmaps, areas
+
+
+@pytest.mark.parametrize("dens,syns,mad", [(1, 1, 0), (1, 1, 3), (2, 1, 1), (1, 3, 0), (2, 2, 0)])
+@pytest.mark.parametrize("kind", ["proximal", "distal"])
+@pytest.mark.parametrize("side,depth,batched", [(17, 1, False), (40, 3, True), (19, 9, False), (132, 1, False)])
+def test_tufts_of_a_few_synapses(dens, syns, mad, kind, side, depth, batched):
+    """Tufts of up to four synapses a cell: folded into the tail (one-synapse
+    ones with every input loaded first), in columns deeper than a warp's
+    group, as a distal tuft that learns, and too many to fold."""
+    src = M.TuftSourceLayer.define("iv").syn_reach(2).prevalence(1)
+    tiny = getattr(M.TuftScheme.basal(), kind)().dens_per_tft(dens).syns_per_den(syns).max_active_dens_l2(mad)
+    other = "distal" if kind == "proximal" else "proximal"
+    big = getattr(M.TuftScheme.basal(), other)().dens_per_tft(4).syns_per_den(16).max_active_dens_l2(1)
+    l2, a2 = _small(side, depth, M.CellScheme.pyramidal().tft(tiny.src_lyr(src)).tft(big.src_lyr(src)))
+    ctx = cortex._Ctx(0)
+    a = cortex.CorticalArea(ctx, M.area_desc("v1", l2, a2, settings_for()), 7)
+    slab = initial_slab(a.plan, 7, scramble_seed=11, clean_flags=True)
+    a.write_slab(slab)
+    b = cortex.Batch(ctx, [a]) if batched else None
+    fr = frames_for(a.plan, 3, 5)
+    for k in range(3):
+        a.write_input(fr[k])
+        (b or a).cycle(1)
+        oracle.intake(a.plan, slab, 0, 0, fr[k])
+        oracle.run(a.plan, slab, None, 1, start_cycle=k)
+        dev = a.read_slab()
+        assert np.array_equal(dev, slab), "cycle %d\n%s" % (k, diff_report(a.plan, dev, slab))
+    if b:
+        b.close()
+    a.close()
+    ctx.close()
