@@ -112,17 +112,42 @@ __device__ __forceinline__ uint8_t inhib_simple_cell(uint8_t* __restrict__ axns,
     int uninhibited = 1;
     int horizon = radius + kInhibHorizOffset;
     int infl_max = horizon * horizon;
+    if constexpr (R > 0) {
+        // A neighbour's influence depends on its ring alone, so each ring's
+        // greatest state decides. Rings weigh less the farther out they lie,
+        // so a neighbour beside the layer may be replaced by the one of its
+        // row in the cell's own column, which lies no farther out and is
+        // held against its own ring as well: no load needs a test.
+        int cu[2 * R + 1];
 #pragma unroll
-    for (int vo = -radius; vo <= radius; vo++) {
-        int uz = max(-radius, -vo - radius), um = min(radius, -vo + radius);
+        for (int k = 0; k < 2 * R + 1; k++) cu[k] = (uint32_t)(u + k - R) < (uint32_t)usz ? k - R : 0;
+        uint32_t most[R + 1] = {};
 #pragma unroll
-        for (int uo = uz; uo <= um; uo++) {
-            int vt = v + (int)(int8_t)vo, ut = u + (int)(int8_t)uo;
-            bool ns = (vt >= 0) & (vt < vsz) & (ut >= 0) & (ut < usz);
-            uint8_t nei = ns ? cs[(uint32_t)s * (uint32_t)(vsz * usz) + (uint32_t)(vt * usz + ut)] : (uint8_t)0;
-            int dist = (abs(vo) + abs(uo) + abs(-vo - uo)) >> 1;
-            int dd = dist - kInhibCenterOffset;
-            uninhibited &= ((int)cel_state * infl_max) >= ((int)nei * (infl_max - dd * dd));
+        for (int vo = -R; vo <= R; vo++) {
+            if ((uint32_t)(v + vo) >= (uint32_t)vsz) continue;
+            const uint8_t* row = cs + (int64_t)c + vo * usz;
+#pragma unroll
+            for (int uo = (vo < 0 ? -vo - R : -R); uo <= (vo < 0 ? R : R - vo); uo++) {
+                const int dist = (abs(vo) + abs(uo) + abs(-vo - uo)) >> 1;
+                most[dist] = max(most[dist], (uint32_t)row[cu[uo + R]]);
+            }
+        }
+#pragma unroll
+        for (int d = 1; d <= R; d++) {
+            const int dd = d - kInhibCenterOffset;
+            uninhibited &= ((int)cel_state * infl_max) >= ((int)most[d] * (infl_max - dd * dd));
+        }
+    } else {
+        for (int vo = -radius; vo <= radius; vo++) {
+            int uz = max(-radius, -vo - radius), um = min(radius, -vo + radius);
+            for (int uo = uz; uo <= um; uo++) {
+                int vt = v + (int)(int8_t)vo, ut = u + (int)(int8_t)uo;
+                bool ns = (vt >= 0) & (vt < vsz) & (ut >= 0) & (ut < usz);
+                uint8_t nei = ns ? cs[(uint32_t)s * (uint32_t)(vsz * usz) + (uint32_t)(vt * usz + ut)] : (uint8_t)0;
+                int dist = (abs(vo) + abs(uo) + abs(-vo - uo)) >> 1;
+                int dd = dist - kInhibCenterOffset;
+                uninhibited &= ((int)cel_state * infl_max) >= ((int)nei * (infl_max - dd * dd));
+            }
         }
     }
     const uint8_t out = (uint8_t)(uninhibited * cel_state);
