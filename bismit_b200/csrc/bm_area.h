@@ -149,6 +149,13 @@ inline void ctx_retain(bm_ctx c) {
 void ctx_release(bm_ctx c);   // frees the context with its last reference
 }  // namespace bm
 
+namespace bm {
+constexpr uint32_t kUpSlots = 4;
+// Frames and outputs of up to this many bytes cross the host link inside the
+// copy kernel of the cycling stream: no copy engine, no event between streams.
+constexpr size_t kDirectBytes = 256 << 10;
+}  // namespace bm
+
 struct bm_area_s {
     using Step = bm::Step;
     bm_ctx ctx = nullptr;
@@ -212,15 +219,23 @@ struct bm_area_s {
     bool front_last = false;      // the latest enqueued cycle used the front stream
     std::vector<bm_sampler_s*> samplers;   // per-cycle readback channels (bm_sampler.cu)
     // Host frames (bm_area_write_input) are copied into a pinned slot during
-    // the call, uploaded on `up` into a device slot while earlier cycles
-    // run, and moved into place on the area's stream. Two slots, each reused
-    // once the area's stream has taken the frame it held (up_taken).
+    // the call. Up to kDirectBytes the intake kernel reads the slot itself,
+    // mapped into the device's address space; a slot is reused once that
+    // kernel has run (up_taken). Larger frames are uploaded from slots 0 and 1
+    // on `up` into a device slot while earlier cycles run, and moved into place
+    // on the area's stream.
     cudaStream_t up = nullptr;
-    uint8_t* up_host[2] = {};
+    uint8_t* up_host[bm::kUpSlots] = {};
+    uint8_t* up_map[bm::kUpSlots] = {};    // the device's address of up_host
     uint8_t* up_dev[2] = {};
-    cudaEvent_t up_loaded[2] = {}, up_taken[2] = {};
-    uint32_t up_next = 0;
+    cudaEvent_t up_loaded[2] = {}, up_taken[bm::kUpSlots] = {};
+    bool up_direct[bm::kUpSlots] = {};     // the slot's last frame was read in place
+    uint32_t up_next = 0, up_next_dev = 0;
     size_t up_cap = 0;
+    // Outputs read back up to kDirectBytes: a kernel writes them here.
+    uint8_t* out_host = nullptr;
+    uint8_t* out_map = nullptr;
+    size_t out_cap = 0;
     // Samplers' device-to-host copies run on `down`, from a device copy of
     // the sampled range taken on the cycling stream.
     cudaStream_t down = nullptr;
