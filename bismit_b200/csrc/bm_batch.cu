@@ -470,7 +470,9 @@ int build_step(bm_ctx ctx, bm_batch_s::StepPlan& p) {
     if (all_ok) {
         // Tile size from the whole step's work, not each area's own: one
         // launch serves every area, so small areas need not cut tiny tiles
-        // to fill the device (the autotuner refines this).
+        // to fill the device (the autotuner refines this): about one tile per
+        // resident CTA, as plan_tuft aims for (12 cycles of three areas joined
+        // by tracts: 1696 us at a fifth of that, 1548 so).
         uint64_t total = 0;
         int sms = 148;
         for (auto& [A, t] : p.tufts) {
@@ -480,9 +482,9 @@ int build_step(bm_ctx ctx, bm_batch_s::StepPlan& p) {
         }
         // A power of two, so that batches rebuilt as areas come and go keep
         // their tiles (and compiled offsets) until the work doubles or halves.
-        uint64_t want = std::min<uint64_t>(65536, std::max<uint64_t>(4096, total / ((uint64_t)sms * 16)));
+        uint64_t want = std::min<uint64_t>(65536, std::max<uint64_t>(4096, total / ((uint64_t)sms * 3)));
         uint32_t target = 4096;
-        while ((uint64_t)target * 2 <= want) target *= 2;
+        while (target < want) target *= 2;
         for (auto& [A, t] : p.tufts) {
             FusedTuft& FT = A->fused.t[st.layer][t];
             // An autotuned choice stays; an area another batch also holds

@@ -107,6 +107,7 @@ struct FusedTuftArgs {
     uint64_t n_units;
     // Tiled form.
     uint32_t tile_w, tile_h, tiles_u, tiles_v, n_tiles;
+    TileSplit split;                    // of n_tiles over the grid
     uint64_t usz_magic;                 // div_magic(u_size), for multi-row tiles
     uint64_t per_slice_magic, tiles_u_magic;   // div_magic of the tiles per slice and per row
     int32_t rv, ru;                     // largest |v|, |u| offset served from the footprint
@@ -500,6 +501,38 @@ __device__ __forceinline__ TileGeo tile_geo(const FusedTuftArgs& A, uint32_t t) 
     g.syn0 = g.cell0 << A.S_l2;
     g.syn_end = (g.cell0 + g.h * g.w) << A.S_l2;
     return g;
+}
+
+// Work item t of a launch: a whole tile, or one of the parts that the tiles of
+// the grid's last round are cut into (TileSplit).
+struct WorkItem {
+    uint32_t tile, part, parts;
+};
+__device__ __forceinline__ WorkItem work_item(const TileSplit& S, uint32_t t) {
+    if (t < S.whole) return {t, 0u, 1u};
+    const uint32_t q = (t - S.whole) / S.parts;
+    return {S.whole + q, t - S.whole - q * S.parts, S.parts};
+}
+// Narrows tile G to part `part` of `parts`, in whole stages; syn0 == syn_end
+// where it has none.
+__device__ __forceinline__ void take_part(const FusedTuftArgs& A, TileGeo& G, uint32_t part, uint32_t parts) {
+    if (parts == 1) return;
+    const uint32_t sb = A.stage_bytes;   // a power of two
+    const uint32_t stages = (G.syn_end - G.syn0 + sb - 1) >> (31 - __clz((int)sb));
+    const uint32_t per = (stages + parts - 1) / parts;
+    G.syn0 = min(G.syn_end, G.syn0 + part * per * sb);
+    G.syn_end = min(G.syn_end, G.syn0 + per * sb);
+}
+
+// Work item t of a one-tuft launch. SPLIT: it has parts (without, the kernel is
+// as it would be with whole tiles only: area_256's cycle 0.7 % shorter).
+template <bool SPLIT>
+__device__ __forceinline__ TileGeo item_geo(const FusedTuftArgs& A, uint32_t t) {
+    if (!SPLIT) return tile_geo(A, t);
+    const WorkItem w = work_item(A.split, t);
+    TileGeo G = tile_geo(A, w.tile);
+    take_part(A, G, w.part, w.parts);
+    return G;
 }
 
 // The position of the 16 synapses at tuft offset `off` in the footprint of
@@ -1086,7 +1119,7 @@ __device__ __forceinline__ bool consume_tile(const FusedTuftArgs& A, const TileG
     consumers_sync();
     const uint32_t SB = stage_syns<MODE, FCLEAN>(A.stage_bytes);
     const uint32_t cpu = A.chunks_per_unit;
-    const uint32_t n_units_tile = cpu > 1 ? G.h * G.w : (G.syn_end - G.syn0 + 511) >> 9;
+    const uint32_t n_units_tile = cpu > 1 ? (G.syn_end - G.syn0) >> A.unit_l2 : (G.syn_end - G.syn0 + 511) >> 9;
     FastCarry C = {0, kNoDen, 0};
     for (uint32_t pos = G.syn0; pos < G.syn_end; pos += SB) {
         const uint32_t cb = ring & kRingBuf;
@@ -1142,7 +1175,7 @@ __device__ __noinline__ void seg_tile(const FusedTuftArgs& A, uint32_t t, uint8_
     fence_proxy_async_smem();   // a later tile's box may overwrite these bytes
 }
 
-template <bool TUFT, int MODE, bool FCLEAN, int GEOM>
+template <bool TUFT, int MODE, bool FCLEAN, int GEOM, bool SPLIT>
 __device__ __forceinline__ void tma_body(const FusedTuftArgs& A, uint8_t* smem, volatile int& s_abort) {
     uint64_t* full = (uint64_t*)(smem + A.ring_off);   // [nst]
     uint64_t* empty = full + A.nst;                    // [nst]
@@ -1158,8 +1191,10 @@ __device__ __forceinline__ void tma_body(const FusedTuftArgs& A, uint8_t* smem, 
         ProducerState ps;
         ps.ctl = A.ctl;
         ps.stall = blockIdx.x == 0 ? A.ctl->stall_stage : 0u;
-        for (uint32_t t = blockIdx.x; t < A.n_tiles && !s_abort; t += gridDim.x)
-            if (!produce_tile<TUFT, MODE, FCLEAN>(A, tile_geo(A, t), stages, full, empty, ps, s_abort)) break;
+        for (uint32_t t = blockIdx.x; t < A.split.items && !s_abort; t += gridDim.x) {
+            const TileGeo G = item_geo<SPLIT>(A, t);
+            if (!produce_tile<TUFT, MODE, FCLEAN>(A, G, stages, full, empty, ps, s_abort)) break;
+        }
         if (s_abort || ps.withheld >= 0) producer_drain(full, A.nst, ps);
         return;
     }
@@ -1167,8 +1202,9 @@ __device__ __forceinline__ void tma_body(const FusedTuftArgs& A, uint8_t* smem, 
     const int32_t rnd = rnd_at(A.rnd_key, cycle_of(A));
     uint32_t ring = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < A.n_tiles; t += gridDim.x) {
-        const TileGeo G = tile_geo(A, t);
+    for (uint32_t t = blockIdx.x; t < A.split.items; t += gridDim.x) {
+        const TileGeo G = item_geo<SPLIT>(A, t);
+        if (SPLIT && G.syn0 == G.syn_end) continue;
         // Every consumer is done with the previous tile; all leave together
         // if any gave up.
         if (consumers_sync_or(!ok || s_abort)) break;
@@ -1207,11 +1243,11 @@ __device__ __forceinline__ uint32_t mode_of(const FusedTuftArgs& A) {
 // (through the call's pointer a 97 x 97 area's cycle was a sixth slower).
 template <bool TUFT, int MODE, bool FCLEAN>
 __device__ __noinline__ void tma_body_general(const FusedTuftArgs& A, uint8_t* smem, volatile int& s_abort) {
-    tma_body<TUFT, MODE, FCLEAN, 0>(A, smem, s_abort);
+    tma_body<TUFT, MODE, FCLEAN, 0, true>(A, smem, s_abort);
 }
 // FORM: 0 the tuft's shape has no specialised consumer (A.geom), 1 it has, 2 it
 // has and the tuft is unaligned.
-template <bool TUFT, int FORM>
+template <bool TUFT, int FORM, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_constant__ FusedTuftArgs A) {
     pdl_begin();
     extern __shared__ __align__(128) uint8_t smem[];
@@ -1221,10 +1257,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_con
     const uint32_t mode = mode_of(A);
     if constexpr (FORM == 0) {
         switch (mode) {
-        case 0: tma_body<TUFT, 0, true, 0>(A, smem, s_abort); break;
-        case 1: tma_body<TUFT, 0, false, 0>(A, smem, s_abort); break;
-        case 2: tma_body<TUFT, 1, true, 0>(A, smem, s_abort); break;
-        default: tma_body<TUFT, 1, false, 0>(A, smem, s_abort); break;
+        case 0: tma_body<TUFT, 0, true, 0, SPLIT>(A, smem, s_abort); break;
+        case 1: tma_body<TUFT, 0, false, 0, SPLIT>(A, smem, s_abort); break;
+        case 2: tma_body<TUFT, 1, true, 0, SPLIT>(A, smem, s_abort); break;
+        default: tma_body<TUFT, 1, false, 0, SPLIT>(A, smem, s_abort); break;
         }
         return;
     }
@@ -1245,16 +1281,16 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_con
     }
     if constexpr (TUFT) {
         switch (A.geom) {
-        case 3: tma_body<TUFT, M, true, 3>(A, smem, s_abort); return;
-        case 4: tma_body<TUFT, M, true, 4>(A, smem, s_abort); return;
-        case 5: tma_body<TUFT, M, true, 5>(A, smem, s_abort); return;
-        case 6: tma_body<TUFT, M, true, 6>(A, smem, s_abort); return;
-        case 7: tma_body<TUFT, M, true, 7>(A, smem, s_abort); return;
-        default: tma_body<TUFT, M, true, 8>(A, smem, s_abort); return;
+        case 3: tma_body<TUFT, M, true, 3, SPLIT>(A, smem, s_abort); return;
+        case 4: tma_body<TUFT, M, true, 4, SPLIT>(A, smem, s_abort); return;
+        case 5: tma_body<TUFT, M, true, 5, SPLIT>(A, smem, s_abort); return;
+        case 6: tma_body<TUFT, M, true, 6, SPLIT>(A, smem, s_abort); return;
+        case 7: tma_body<TUFT, M, true, 7, SPLIT>(A, smem, s_abort); return;
+        default: tma_body<TUFT, M, true, 8, SPLIT>(A, smem, s_abort); return;
         }
     } else {
-        if (A.geom == 1) tma_body<TUFT, 0, true, 1>(A, smem, s_abort);
-        else tma_body<TUFT, 0, true, 2>(A, smem, s_abort);
+        if (A.geom == 1) tma_body<TUFT, 0, true, 1, SPLIT>(A, smem, s_abort);
+        else tma_body<TUFT, 0, true, 2, SPLIT>(A, smem, s_abort);
     }
 }
 
@@ -1267,11 +1303,12 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_con
 // the stores of a stage, and nothing needs copying per job. Every job of a
 // launch shares the ring geometry (nst, stage_stride, ring_off).
 // As many argument blocks as fit the 32 KB kernel parameter limit.
-constexpr uint32_t kMaxBatchJobs = (32764 - 16) / (sizeof(FusedTuftArgs) + 4) - 1;
+constexpr uint32_t kMaxBatchJobs = (32764 - 32) / (sizeof(FusedTuftArgs) + 4) - 1;
 
 struct BatchParams {
     FusedTuftArgs jobs[kMaxBatchJobs];
     uint32_t tile0[kMaxBatchJobs + 1];
+    TileSplit split;   // of all jobs' tiles over the grid
     uint32_t n_jobs, nst, ring_off;
 };
 static_assert(sizeof(BatchParams) <= 32764, "batched tuft parameter block exceeds the kernel parameter limit");
@@ -1309,7 +1346,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_batch(const __grid_c
         uint32_t cur = 0xFFFFFFFFu, mode = 0;
         ProducerState ps;
         AreaCtl* ctl = nullptr;
-        for (uint32_t t = blockIdx.x; t < n_tiles && !s_abort; t += gridDim.x) {
+        for (uint32_t i = blockIdx.x; i < P.split.items && !s_abort; i += gridDim.x) {
+            const WorkItem w = work_item(P.split, i);
+            const uint32_t t = w.tile;
             const uint32_t j = job_of(P, t);
             const FusedTuftArgs& A = P.jobs[j];
             if (j != cur) {
@@ -1320,9 +1359,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_batch(const __grid_c
                 // takes a job's first tile withholds the job area's
                 // stall_stage-th stage from that tile on.
                 ps.ctl = ctl;
-                if (t == P.tile0[j] && ctl->stall_stage) ps.stall = ps.issued + ctl->stall_stage;
+                if (t == P.tile0[j] && w.part == 0 && ctl->stall_stage) ps.stall = ps.issued + ctl->stall_stage;
             }
-            const TileGeo G = tile_geo(A, t - P.tile0[j]);
+            TileGeo G = tile_geo(A, t - P.tile0[j]);
+            take_part(A, G, w.part, w.parts);
             bool ok;
             if constexpr (MIS) {
                 if (mode) continue;   // no stages: the consumers take the tile in the windowed form
@@ -1342,7 +1382,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_batch(const __grid_c
     uint32_t cur = 0xFFFFFFFFu, mode = 0, ring = 0;
     int32_t rnd = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+    for (uint32_t i = blockIdx.x; i < P.split.items; i += gridDim.x) {
+        const WorkItem w = work_item(P.split, i);
+        const uint32_t t = w.tile;
         const uint32_t j = job_of(P, t);
         const FusedTuftArgs& A = P.jobs[j];
         // Every consumer is done with the previous tile; all leave together
@@ -1353,7 +1395,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_batch(const __grid_c
             mode = mode_of(A);
             rnd = rnd_at(A.rnd_key, cycle_of(A));
         }
-        const TileGeo G = tile_geo(A, t - P.tile0[j]);
+        TileGeo G = tile_geo(A, t - P.tile0[j]);
+        take_part(A, G, w.part, w.parts);
+        if (G.syn0 == G.syn_end) continue;
 #define BM_CONSUME(M, FC, GM)                                                                                   \
     ok = consume_tile<TUFT, M, FC, GM>(A, G, halo, stages, full, empty, fp_full, ring, lane, wib, rnd, s_abort)
         if constexpr (MIS) {
@@ -1505,10 +1549,26 @@ int device_sms() {
 // The one-tuft kernel of a layer kind, for a shape with a specialised consumer
 // or without, or for an unaligned tuft.
 using TmaKernel = void (*)(FusedTuftArgs);
-TmaKernel tma_kernel(bool pyr, bool fast, bool mis) {
-    if (pyr) return mis ? k_fused_tuft_tma<true, 2> : fast ? k_fused_tuft_tma<true, 1> : k_fused_tuft_tma<true, 0>;
-    return fast ? k_fused_tuft_tma<false, 1> : k_fused_tuft_tma<false, 0>;
+TmaKernel tma_kernel(bool pyr, bool fast, bool mis, bool split) {
+    if (mis) return k_fused_tuft_tma<true, 2, true>;
+    if (!fast) return pyr ? k_fused_tuft_tma<true, 0, true> : k_fused_tuft_tma<false, 0, true>;
+    if (split) return pyr ? k_fused_tuft_tma<true, 1, true> : k_fused_tuft_tma<false, 1, true>;
+    return pyr ? k_fused_tuft_tma<true, 1, false> : k_fused_tuft_tma<false, 1, false>;
 }
+
+// How n tiles of up to `stages` stages share `ctas` resident CTAs: the tiles of
+// the last round are cut into parts while there are fewer of them than CTAs, so
+// that it does not leave most of the device idle (900 tiles of a 150 x 150 x 3
+// instance over 444 CTAs: the last 12 took as long as the 888 before them).
+TileSplit tile_split(uint32_t n, uint32_t ctas, uint32_t stages) {
+    const uint32_t rem = n % ctas;
+    TileSplit S;
+    S.whole = n - rem;
+    S.parts = rem ? std::max<uint32_t>(1, std::min(ctas / rem, stages)) : 1;
+    S.items = S.whole + rem * S.parts;
+    return S;
+}
+uint32_t stages_of(uint64_t syns, uint32_t stage) { return (uint32_t)((syns + stage - 1) / stage); }
 
 // Launch parameters of tuft t of data layer i (gidx left null). `target` is
 // the synapses per tile to aim for (0: chosen from the tuft's size);
@@ -1562,7 +1622,14 @@ void plan_tuft_form(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t
     const uint32_t cpu = S > 512 ? S / 512 : 1;
     const uint32_t SB = kWarps * cpu * 512;
     const uint64_t n_syn = (uint64_t)L.cells * S;
-    uint64_t target = std::min<uint64_t>(kMaxTileSyns, std::max<uint64_t>(4096, n_syn / ((uint64_t)sms * 16)));
+    // One tile per resident CTA where that is not too large a tile: each tile
+    // starts with its footprint's load and two barriers. (120 x 120 x 2 with
+    // 8 x 32 tufts, 24 cycles: 727 us at a 16th of an SM's share, 630 at a
+    // third; three areas of up to 192 x 192 x 2 in a batch, 12 cycles: 1696 and
+    // 1551.) Spiny stellate tufts keep smaller ones: they head the cycle's chain
+    // beside another tuft's tiles (256 x 256 live: 334 us a frame, 346).
+    const uint64_t share = (uint64_t)sms * (L.kind == BM_LYR_PYRAMIDAL ? 3 : 16);
+    uint64_t target = std::min<uint64_t>(kMaxTileSyns, std::max<uint64_t>(4096, (n_syn + share - 1) / share));
     if (target_syns) target = target_syns;
     const uint64_t cells = std::max<uint64_t>(1, target / S);
     const uint32_t vs = P.slc_v_scale[lo], us = P.slc_u_scale[lo];
@@ -1663,15 +1730,21 @@ void plan_tuft_form(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t
     for (uint32_t k = 0; k < nrec; k++) FT.src_idz[k] = P.slc_axn_idz[lo + k];
     // Persistent grid: as many CTAs as fit on the device at once.
     const bool pyr = L.kind == BM_LYR_PYRAMIDAL;
-    auto kern = tma_kernel(pyr, consumer_shape(FT, S, spd, pyr) != 0, FT.mis != 0);
+    const bool fast = consumer_shape(FT, S, spd, pyr) != 0;
     // The cap is a property of the kernel, shared by every area on the device:
-    // set it to the largest footprint any tuft may plan, never lower.
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+    // set it to the largest footprint any tuft may plan, never lower. Both
+    // kernels of the tuft (its split is not known yet) fit the same CTAs.
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, FT.smem) != cudaSuccess)
-        per_sm = 1;
+    for (bool split : {false, true}) {
+        auto kern = tma_kernel(pyr, fast, FT.mis != 0, split);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kThreads, FT.smem) != cudaSuccess) n = 1;
+        per_sm = per_sm ? std::min(per_sm, n) : n;
+    }
     const uint64_t n_tiles = (uint64_t)L.depth * ((L.u_size + W - 1) / W) * ((L.v_size + H - 1) / H);
-    FT.grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(n_tiles, (uint64_t)sms * std::max(per_sm, 1)));
+    FT.split = tile_split((uint32_t)n_tiles, (uint32_t)(sms * std::max(per_sm, 1)), stages_of((uint64_t)W * H * S, SB));
+    FT.grid = std::max<uint32_t>(1, std::min<uint32_t>(FT.split.items, (uint32_t)(sms * std::max(per_sm, 1))));
 }
 
 }  // namespace
@@ -1948,6 +2021,7 @@ void make_args(FusedTuftArgs& A, const FusedArea& F, const uint8_t* axns, const 
         A.tiles_u = (L.u_size + FT.tile_w - 1) / FT.tile_w;
         A.tiles_v = (L.v_size + FT.tile_h - 1) / FT.tile_h;
         A.n_tiles = L.depth * A.tiles_u * A.tiles_v;
+        A.split = FT.split;
         A.usz_magic = div_magic(L.u_size);
         A.per_slice_magic = div_magic(A.tiles_u * A.tiles_v);
         A.tiles_u_magic = div_magic(A.tiles_u);
@@ -1994,7 +2068,7 @@ void launch_fused_tuft(const FusedArea& F, const uint8_t* axns, const SliceRec* 
     }
     const bool tuft = L.kind == BM_LYR_PYRAMIDAL;
     if (FT.tiled) {
-        auto kern = tma_kernel(tuft, A.geom != 0, FT.mis != 0);
+        auto kern = tma_kernel(tuft, A.geom != 0, FT.mis != 0, FT.split.parts > 1);
         launch_pdl(kern, FT.grid, kThreads, FT.smem, s, A);
     } else {
         uint64_t want = (A.n_units + kWarps - 1) / kWarps;
@@ -2072,7 +2146,7 @@ int prepare_fused_batch(FusedBatch& B, const std::vector<FusedJob>& jobs, const 
             }
             std::memset(P, 0, sizeof *P);
             const size_t n = std::min<size_t>(kMaxBatchJobs, cls.size() - j0);
-            uint32_t total = 0;
+            uint32_t total = 0, most = 1;   // tiles, and a tile's most stages
             for (size_t j = 0; j < n; j++) {
                 const FusedJob& J = *cls[j0 + j];
                 make_args(P->jobs[j], *J.F, J.axns, J.slices, *J.L, J.layer, J.t, J.ctl, J.ssc_soma);
@@ -2080,6 +2154,8 @@ int prepare_fused_batch(FusedBatch& B, const std::vector<FusedJob>& jobs, const 
                 P->jobs[j].stage_stride = stride;
                 P->jobs[j].ring_off = (uint32_t)ring_off;
                 P->tile0[j] = total;
+                const FusedTuft& FT = J.F->t[J.layer][J.t];
+                most = std::max(most, stages_of(((uint64_t)FT.tile_w * FT.tile_h) << P->jobs[j].S_l2, FT.stage_bytes));
                 total += P->jobs[j].n_tiles;
             }
             P->tile0[n] = total;
@@ -2087,7 +2163,8 @@ int prepare_fused_batch(FusedBatch& B, const std::vector<FusedJob>& jobs, const 
             P->nst = nst;
             P->ring_off = (uint32_t)ring_off;
             B.params.push_back(P);
-            B.grids.push_back((uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(total, (uint64_t)sms * std::max(per_sm, 1))));
+            P->split = tile_split(total, sms * (uint32_t)std::max(per_sm, 1), most);
+            B.grids.push_back(std::max<uint32_t>(1, std::min<uint32_t>(P->split.items, sms * (uint32_t)std::max(per_sm, 1))));
             B.smems.push_back((uint32_t)smem);
             B.mis.push_back(mis);
             B.n_tiles += total;

@@ -9,6 +9,12 @@
 
 namespace bm {
 
+// A launch's work items: `whole` tiles, then the remaining ones in `parts` parts
+// each, `items` in all.
+struct TileSplit {
+    uint32_t whole = 0, parts = 1, items = 0;
+};
+
 // Launch parameters of the fused kernel for one tuft.
 struct FusedTuft {
     bool ok = false;         // the fused kernel applies to this tuft
@@ -25,6 +31,7 @@ struct FusedTuft {
                                 // specialised consumer only)
     uint32_t smem = 0;       // dynamic shared memory per CTA
     uint32_t grid = 1;       // persistent grid size
+    TileSplit split;
     uint32_t nst = 2;        // TMA pipeline stages
     uint32_t stage_bytes = 0;
     uint32_t ring_off = 0;   // ring offset in dynamic shared memory (the footprint is at 0)

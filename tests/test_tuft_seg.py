@@ -23,6 +23,12 @@ SHAPES = [
     ("unaligned_512b", lambda: configs.instance_area(29, 3, 8, 64), True),
     ("unaligned_512c", lambda: configs.instance_area(66, 4, 16, 32), True),
     ("unaligned_1024b", lambda: configs.instance_area(37, 3, 16, 64), True),
+    # Tiles of several stages, the last round's cut into parts.
+    ("split_512", lambda: configs.instance_area(100, 1, 16, 32), True),
+    ("split_512_unaligned", lambda: configs.instance_area(101, 1, 16, 32), True),
+    ("split_1024", lambda: configs.instance_area(96, 2, 16, 64), True),
+    ("split_1024_unaligned", lambda: configs.instance_area(90, 2, 16, 64), True),
+    ("split_general", lambda: configs.instance_area(100, 2, 2, 128), True),
     ("wide_16", lambda: configs.instance_area(321, 3, 1, 8), False),           # 16-byte windows
     ("unaligned_16", lambda: configs.instance_area(33, 2, 1, 16), False),
     ("odd_21", lambda: configs.instance_area(32, 2, 3, 7), False),
@@ -64,7 +70,7 @@ def test_matches_oracle(label, mk, fused, clean_flags):
     ctx.close()
 
 
-@pytest.mark.parametrize("sides", [(19, 33, 21), (65, 71, 30)])
+@pytest.mark.parametrize("sides", [(19, 33, 21), (65, 71, 30), (100, 96, 40), (101, 90, 39)])
 def test_batched_matches_alone(sides):
     ctx = cortex._Ctx(0)
     descs = [_desc(lambda s=s: configs.instance_area(s, 1 + s % 2, 16, 32), settings_for()) for s in sides]
