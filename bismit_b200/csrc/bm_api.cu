@@ -102,9 +102,17 @@ void push_layer_learn(const bm_area_s* A, uint32_t i, std::vector<Step>& out) {
     }
 }
 
-// Tuft t of data layer i may fold into its layer's tail, a thread per cell.
+// Tuft t of data layer i may fold into its layer's tail, a thread per cell: the
+// tail writes the layer's own axons, so the tuft must read none of them (one
+// thread's output would race another's gather).
 bool cell_tuft(const bm_area_s* A, uint32_t i, uint32_t t) {
-    return !A->fused.t[i][t].ok && A->plan.layers[i].tufts[t].syns_per_tft <= kCellTuftSyns;
+    const bm_layer_plan& L = A->plan.layers[i];
+    if (A->fused.t[i][t].ok || L.tufts[t].syns_per_tft > kCellTuftSyns || ((A->foreign_src[i] >> t) & 1)) return false;
+    for (uint32_t k = 0; k < L.tufts[t].n_src_uniq; k++) {
+        const uint32_t s = L.tufts[t].src_uniq_slc_ids[k];
+        if (s >= L.base_axn_slc && s < L.base_axn_slc + L.depth) return false;
+    }
+    return true;
 }
 
 // Slices of data layer i are plain: unscaled, unshifted and laid out back to
@@ -500,6 +508,7 @@ void bm::note_sources(bm_area_s* A, uint32_t i, uint64_t b, uint64_t e, const ui
     if (next == A->foreign_src[i]) return;
     A->foreign_src[i] = next;
     A->access_version++;
+    area_steps(A, A->steps, cell_tuft_cells(A) <= kFoldCellTufts);   // a folded tuft may have to leave the tail
     schedule_area(A);
 }
 

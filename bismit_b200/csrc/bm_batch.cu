@@ -817,6 +817,27 @@ int after_cycle(bm_batch_s* B, cudaStream_t s) {
     return BM_OK;
 }
 
+std::string step_key(const bm_batch_s::StepPlan& p);
+
+// The plan made anew, its autotuned launch shapes kept.
+int rebuild_plan(bm_batch_s* B) {
+    const cudaError_t e = cudaStreamSynchronize(B->stream());   // the queued cycles use the old tables
+    if (e != cudaSuccess) return cuda_err(e, "batched plan");
+    std::map<std::string, BatchShape> shapes;
+    for (const auto& p : B->plan)
+        if (p.form == bm_batch_s::F_FUSED) shapes[step_key(p)] = p.shape;
+    int rc = build_plan(B);
+    for (auto& p : B->plan) {
+        const auto hit = p.form == bm_batch_s::F_FUSED ? shapes.find(step_key(p)) : shapes.end();
+        if (rc != BM_OK || hit == shapes.end()) continue;
+        p.shape = hit->second;
+        free_fused_batch(p.fb);
+        rc = build_fused(p);
+    }
+    count_launches(B);
+    return rc;
+}
+
 int run_cycles(bm_batch_s* B, const void* frames, uint32_t n_cycles, bool refuse_after_errors = true) {
     if (B->detached) return set_err(BM_ERR_INVALID, "an area of this batch was destroyed");
     // An area whose earlier cycle ended with device error bits stops the batch
@@ -831,8 +852,16 @@ int run_cycles(bm_batch_s* B, const void* frames, uint32_t n_cycles, bool refuse
     for (size_t a = 0; a < B->areas.size(); a++)
         if (a >= B->versions.size() || B->areas[a]->access_version != B->versions[a]) {
             B->drop_graph();
-            const int rc = schedule_side(B);
+            // A folded tuft of a few synapses may have to leave its tail (or
+            // may go back): then the steps change, else only their streams.
+            bool tiny = false;
+            for (bm_area A : B->areas)
+                for (uint32_t i = 0; i < A->plan.n_layers; i++)
+                    for (uint32_t t = 0; t < A->plan.layers[i].n_tufts; t++)
+                        tiny |= !A->fused.t[i][t].ok && A->plan.layers[i].tufts[t].syns_per_tft <= kCellTuftSyns;
+            const int rc = tiny ? rebuild_plan(B) : schedule_side(B);
             if (rc != BM_OK) return rc;
+            for (bm_area A : B->areas) run_pending_verifies(A, s);
             break;
         }
     k_batch_begin<<<1, 1, 0, s>>>(B->d_bctl, (const uint8_t*)frames, B->frame_bytes);

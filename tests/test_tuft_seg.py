@@ -187,3 +187,41 @@ def test_tufts_of_a_few_synapses(dens, syns, mad, kind, side, depth, batched):
         b.close()
     a.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("batched", [False, True])
+@pytest.mark.parametrize("syns", [1, 2])
+def test_few_synapses_from_the_layers_own_axons(syns, batched):
+    """A tuft of a few synapses that reads the axons its layer's tail writes, by
+    its pool or because the caller wrote such sources, does not run inside that
+    tail."""
+    own = M.TuftSourceLayer.define("iii").syn_reach(5).prevalence(1)
+    iv = M.TuftSourceLayer.define("iv").syn_reach(5).prevalence(1)
+
+    def tuft(kind, src):
+        return getattr(M.TuftScheme.basal(), kind)().dens_per_tft(1).syns_per_den(syns).max_active_dens_l2(0).src_lyr(src)
+
+    for srcs in ((iv, own), (iv, iv)):
+        l2, a2 = _small(70, 2, M.CellScheme.pyramidal().tft(tuft("proximal", srcs[0])).tft(tuft("distal", srcs[1])))
+        ctx = cortex._Ctx(0)
+        a = cortex.CorticalArea(ctx, M.area_desc("v1", l2, a2, settings_for()), 7)
+        slab = initial_slab(a.plan, 7, scramble_seed=11, clean_flags=True)
+        a.write_slab(slab)
+        b = cortex.Batch(ctx, [a]) if batched else None
+        fr = frames_for(a.plan, 12, 5, active=0.2)
+        for k in range(12):
+            if k == 4 and srcs[1] is iv:   # the layer's own slices, from here on
+                last = a.plan.layers[1]
+                off = int(last.buf_off[F.BUF["syn_src_slc_ids"]])
+                slab[off:off + int(last.n_syns)] = int(last.base_axn_slc) + np.arange(int(last.n_syns)) % 2
+                a.write("syn_src_slc_ids", slab[off:off + int(last.n_syns)], layer=1)
+            a.write_input(fr[k])
+            (b or a).cycle(1)
+            oracle.intake(a.plan, slab, 0, 0, fr[k])
+            oracle.run(a.plan, slab, None, 1, start_cycle=k)
+            dev = a.read_slab()
+            assert np.array_equal(dev, slab), "cycle %d\n%s" % (k, diff_report(a.plan, dev, slab))
+        if b:
+            b.close()
+        a.close()
+        ctx.close()
