@@ -1212,9 +1212,17 @@ int read_back(bm_area_s* A, const uint8_t* src, uint8_t* dst, size_t len) {
         if (A->out_host) cudaFreeHost(A->out_host);
         A->out_host = A->out_map = nullptr;
         A->out_cap = 0;
-        CU(cudaHostAlloc((void**)&A->out_host, len, cudaHostAllocMapped | cudaHostAllocPortable));
-        CU(cudaHostGetDevicePointer((void**)&A->out_map, A->out_host, 0));
-        A->out_cap = len;
+        if (cudaHostAlloc((void**)&A->out_host, len, cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) {
+            CU(cudaHostGetDevicePointer((void**)&A->out_map, A->out_host, 0));
+            A->out_cap = len;
+        } else {
+            cudaGetLastError();   // no page-locked memory to be had: a plain copy below
+        }
+    }
+    if (A->out_cap < len) {
+        CU(cudaMemcpyAsync(dst, src, len, cudaMemcpyDeviceToHost, A->stream()));
+        CU(cudaStreamSynchronize(A->stream()));
+        return BM_OK;
     }
     CopyPieces P = {};
     P.dst[0] = A->out_map;

@@ -1140,7 +1140,7 @@ __device__ __forceinline__ bool consume_tile(const FusedTuftArgs& A, const TileG
                                                                    pos, lane, wib, C);
         // The buffer is released after the finish: released before it, the
         // loads run further ahead and the cycle is slower (area_256 0.296 ms
-        // against 0.270, same box).
+        // against 0.270).
         if constexpr (GEOM != 0) {
             constexpr uint32_t LPD = 1u << (geom_spd_l2(GEOM) - 4);
             if (C.old >> 16 >= LPD || pos + SB >= G.syn_end)

@@ -117,8 +117,8 @@ struct FusedJob {
 struct FusedBatch {
     bool ok = false;             // every job is tiled and the ring fits: batched launches serve them all
     bool tuft = false;           // pyramidal layer
-    std::vector<void*> params;   // host parameter blocks, one launch each (up to 80 jobs of one
-    std::vector<uint32_t> grids; // stage geometry per launch)
+    std::vector<void*> params;   // host parameter blocks, one launch each (jobs of one
+    std::vector<uint32_t> grids; // stage geometry, as many as a block holds)
     std::vector<uint32_t> smems;
     std::vector<uint8_t> mis;    // launch k's jobs are unaligned tufts
     uint32_t n_jobs = 0, n_tiles = 0;

@@ -107,7 +107,7 @@ __global__ void k_tft_dst_mtp(const uint8_t* __restrict__ axns, DevLayer L, uint
 }
 
 // Tufts of at most kCellTuftSyns synapses a cell, a thread per cell: 28,800
-// one-synapse cells take 7.9 us cold, in k_tuft_seg's blocks 15.6 us (57 of
+// one-synapse cells take 4.7 us cold, in k_tuft_seg's blocks 15.6 us (57 of
 // them, each walking four cells a thread through its three steps).
 __global__ void k_tuft_cells(const uint8_t* __restrict__ axns, const SliceRec* __restrict__ slices, DevLayer L,
                              uint32_t t, const AreaCtl* ctl) {

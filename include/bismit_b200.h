@@ -497,7 +497,7 @@ int bm_area_inject_stall(bm_area area, uint32_t stage);
 typedef struct bm_tuft_form {
     uint32_t fused;            /* the fused tuft kernel runs it                        */
     uint32_t tiled;            /* it gathers from a shared-memory axon footprint       */
-    uint32_t consumer;         /* compile-time specialised consumer shape (1..7), 0 =
+    uint32_t consumer;         /* compile-time specialised consumer shape (1..8), 0 =
                                   the general one                                      */
     uint32_t sources_outside;  /* a source lies outside the footprint: checked gathers */
     uint32_t flags_foreign;    /* a flag byte has bits besides SYN_PREV_ACTIVE: flags
