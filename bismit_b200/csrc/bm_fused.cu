@@ -771,8 +771,9 @@ namespace {
 // the activity rating and the cell's reduction. Instead the warp takes LPD
 // units, lane l keeping the sums of its dendrite of unit l % LPD, and finishes
 // them together: 16 x 32 cells two at a time, 282 warp instructions per 512
-// synapses in place of 334. area_256's cycle 0.286 -> 0.272 ms (5.9 TB/s
-// moved), the three-area hierarchy's 0.174 -> 0.148, 24 instances' 0.473 ->
+// synapses in place of 334 (both with 16-bit offsets; source codes take 326 to
+// 358). area_256's cycle 0.286 -> 0.272 ms (0.260 with the codes), the
+// three-area hierarchy's 0.174 -> 0.148, 24 instances' 0.473 ->
 // 0.441.
 struct FastCarry {
     uint32_t acc;   // raw sum << 16 | sum of the states with non-negative strength
