@@ -132,33 +132,35 @@ bool layer_plain(const bm_area_plan& P, uint32_t i) {
 }
 
 // Brings steps that fuse next to one another, where the order between them does
-// not show.
-//  * A smoother touches its layer's cell activities and energies only. On a
-//    pyramidal layer only a basket inhibition does too, so without one it goes
-//    ahead of the layer's tufts; on a spiny stellate layer learning does not,
-//    so it goes behind that.
+// not show: a step moves only past steps whose accesses do not conflict with
+// its own.
+//  * A smoother stands between steps that fuse. On a pyramidal layer it goes
+//    ahead of the layer's tufts, on a spiny stellate layer behind the layer's
+//    learning, unless a step in between touches activities or energies too (a
+//    basket inhibition): then it stays.
 //  * A pyr_output that an inhib_intra_column of the same layer follows wrote
 //    every axon of the layer, and the intra-column step writes them all again
 //    with nothing in between reading them: it is left out.
 void order_steps(const bm_area_s* A, std::vector<Step>& v) {
     const bm_area_plan& P = A->plan;
+    // Step k may run before or after all of steps [b, e).
+    auto free_of = [&](size_t k, size_t b, size_t e) {
+        const StepAccess a = step_access(A, v[k]);
+        for (size_t j = b; j < e; j++)
+            if (conflict(a, step_access(A, v[j]))) return false;
+        return true;
+    };
     for (size_t k = 0; k < v.size(); k++) {
         if (v[k].kind != ST_SMOOTH || P.layers[v[k].layer].kind != BM_LYR_PYRAMIDAL) continue;
-        bool basket = false;
-        for (size_t j = 0; j < k; j++)
-            basket |= v[j].layer == v[k].layer && (v[j].kind == ST_INHIB_SIMPLE || v[j].kind == ST_INHIB_PASS);
-        if (basket) continue;
         size_t j = 0;
         while (j < k && (v[j].layer != v[k].layer || v[j].kind == ST_SMOOTH || v[j].kind == ST_FILTER)) j++;
-        std::rotate(v.begin() + j, v.begin() + k, v.begin() + k + 1);
+        if (free_of(k, j, k)) std::rotate(v.begin() + j, v.begin() + k, v.begin() + k + 1);
     }
     for (size_t k = v.size(); k-- > 0;) {
         if (v[k].kind != ST_SMOOTH || P.layers[v[k].layer].kind == BM_LYR_PYRAMIDAL) continue;
-        for (size_t j = k + 1; j < v.size(); j++)
-            if (v[j].kind == ST_SSC_MTP && v[j].layer == v[k].layer) {
-                std::rotate(v.begin() + k, v.begin() + k + 1, v.begin() + j + 1);
-                break;
-            }
+        size_t j = k + 1;
+        while (j < v.size() && (v[j].kind != ST_SSC_MTP || v[j].layer != v[k].layer)) j++;
+        if (j < v.size() && free_of(k, k + 1, j + 1)) std::rotate(v.begin() + k, v.begin() + k + 1, v.begin() + j + 1);
     }
     for (size_t k = 0; k + 1 < v.size(); k++)
         if (v[k].kind == ST_PYR_OUTPUT && v[k + 1].kind == ST_INTRA_COL && v[k].layer == v[k + 1].layer)
@@ -414,7 +416,7 @@ bm::StepAccess bm::step_access(const bm_area_s* A, const Step& st, int t) {
         if ((A->foreign_src[i] >> tt) & 1) a.ax_r.set();   // sources anywhere: any slice
         else tuft_sources(P, i, tt, a.ax_r);
         a.tf_r = a.tf_w = tuft_bit(i, tt);
-        if (st.arg & 1) a.ce_r = a.ce_w = 1u << i;          // with the folded ssc_cycle
+        if (st.arg & 1) a.ce_r = a.ce_w = a.ae_r = a.ae_w = 1u << i;   // with the folded ssc_cycle
         break;
     }
     case ST_TUFTS_PLAIN:
@@ -427,15 +429,17 @@ bm::StepAccess bm::step_access(const bm_area_s* A, const Step& st, int t) {
     case ST_PYR_CYCLE:
         a.tf_r = layer_tufts(P, i);
         a.ce_r = a.ce_w = 1u << i;
+        if (st.kind == ST_SSC_CYCLE) a.ae_r = a.ae_w = 1u << i;
         break;
     case ST_INHIB_SIMPLE:
     case ST_INHIB_PASS:
-        a.ce_r = a.ce_w = 1u << i;
+        a.ce_r = a.ce_w = a.ae_r = a.ae_w = 1u << i;
         layer_axons(P, i, a.ax_w);
         break;
     case ST_INHIB_MTP:
     case ST_SSC_MTP:
         a.ce_r = a.ce_w = 1u << i;
+        if (st.kind == ST_INHIB_MTP) a.ae_r = a.ae_w = 1u << i;
         layer_axons(P, i, a.ax_w);
         a.ax_r = a.ax_w;
         a.tf_r = a.tf_w = layer_tufts(P, i);
@@ -446,7 +450,7 @@ bm::StepAccess bm::step_access(const bm_area_s* A, const Step& st, int t) {
         layer_axons(P, i, a.ax_w);
         break;
     case ST_SMOOTH:
-        a.ce_r = a.ce_w = 1u << i;
+        a.ae_r = a.ae_w = 1u << i;
         break;
     case ST_FILTER: {
         // Reads the chain's own buffers, which nothing else in a cycle touches.

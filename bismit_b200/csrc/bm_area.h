@@ -71,17 +71,20 @@ struct Step {
 
 // What a step of one area reads and writes, at the granularity its kernels
 // touch: axon slices, the synapse / dendrite / cell-tuft arrays of one tuft of
-// a layer, and the cell arrays of a layer. Two steps of an area whose accesses
-// do not conflict may run concurrently.
+// a layer, the cell arrays of a layer, and of these the activities and energies
+// apart (all that a smoother touches). Two steps of an area whose accesses do
+// not conflict may run concurrently, or in either order.
 struct StepAccess {
     std::bitset<BM_MAX_SLICES> ax_r, ax_w;
     uint64_t tf_r = 0, tf_w = 0;   // bit layer * BM_MAX_TUFTS + tuft
-    uint32_t ce_r = 0, ce_w = 0;   // bit layer
+    uint32_t ce_r = 0, ce_w = 0;   // bit layer: cell states and flags
+    uint32_t ae_r = 0, ae_w = 0;   // bit layer: cell activities and energies
     bool all = false;              // touches everything (regrowth, the cycle end)
     StepAccess& operator|=(const StepAccess& o) {
         ax_r |= o.ax_r; ax_w |= o.ax_w;
         tf_r |= o.tf_r; tf_w |= o.tf_w;
         ce_r |= o.ce_r; ce_w |= o.ce_w;
+        ae_r |= o.ae_r; ae_w |= o.ae_w;
         all = all || o.all;
         return *this;
     }
@@ -91,6 +94,7 @@ inline bool conflict(const StepAccess& a, const StepAccess& b) {
     if ((a.ax_w & (b.ax_r | b.ax_w)).any() || (b.ax_w & a.ax_r).any()) return true;
     if ((a.tf_w & (b.tf_r | b.tf_w)) || (b.tf_w & a.tf_r)) return true;
     if ((a.ce_w & (b.ce_r | b.ce_w)) || (b.ce_w & a.ce_r)) return true;
+    if ((a.ae_w & (b.ae_r | b.ae_w)) || (b.ae_w & a.ae_r)) return true;
     return false;
 }
 
