@@ -229,6 +229,13 @@ struct bm_batch_s {
         // Profiling (eager cycles only): launches and device milliseconds.
         uint64_t prof_n = 0;
         double prof_ms = 0;
+        uint32_t prof_kind() const { return form == F_FUSED ? 1000u + st.kind : st.kind; }
+    };
+    // A profiled step the plan had before it was made anew.
+    struct Prof {
+        uint32_t kind, layer, idx, n_areas;
+        uint64_t n;
+        double ms;
     };
     bm_ctx ctx = nullptr;
     std::vector<bm_area> areas;          // every area, in batch order
@@ -236,7 +243,8 @@ struct bm_batch_s {
     uint32_t plan_launches = 0;
     bool profiling = false;
     struct Rec { size_t step; cudaEvent_t a, b; };
-    std::vector<Rec> pending;
+    std::vector<Rec> pending;            // steps of the present plan
+    std::vector<Prof> retired;           // profiled steps the present plan has no longer
     std::vector<cudaEvent_t> pool;
     cudaEvent_t ev() {
         if (!pool.empty()) { cudaEvent_t e = pool.back(); pool.pop_back(); return e; }
@@ -819,15 +827,28 @@ int after_cycle(bm_batch_s* B, cudaStream_t s) {
 
 std::string step_key(const bm_batch_s::StepPlan& p);
 
-// The plan made anew, its autotuned launch shapes kept.
+// The plan made anew, its autotuned launch shapes and its profile kept.
 int rebuild_plan(bm_batch_s* B) {
     const cudaError_t e = cudaStreamSynchronize(B->stream());   // the queued cycles use the old tables
     if (e != cudaSuccess) return cuda_err(e, "batched plan");
+    // The records of profiled cycles name steps by their place in the old plan.
+    B->drain_profile();
     std::map<std::string, BatchShape> shapes;
-    for (const auto& p : B->plan)
+    for (const auto& p : B->plan) {
         if (p.form == bm_batch_s::F_FUSED) shapes[step_key(p)] = p.shape;
+        if (p.prof_n)
+            B->retired.push_back({p.prof_kind(), p.st.layer, p.st.idx, (uint32_t)p.areas.size(), p.prof_n, p.prof_ms});
+    }
     int rc = build_plan(B);
     for (auto& p : B->plan) {
+        const auto was = std::find_if(B->retired.begin(), B->retired.end(), [&](const bm_batch_s::Prof& q) {
+            return q.kind == p.prof_kind() && q.layer == p.st.layer && q.idx == p.st.idx;
+        });
+        if (was != B->retired.end()) {
+            p.prof_n = was->n;
+            p.prof_ms = was->ms;
+            B->retired.erase(was);
+        }
         const auto hit = p.form == bm_batch_s::F_FUSED ? shapes.find(step_key(p)) : shapes.end();
         if (rc != BM_OK || hit == shapes.end()) continue;
         p.shape = hit->second;
@@ -835,6 +856,7 @@ int rebuild_plan(bm_batch_s* B) {
         rc = build_fused(p);
     }
     count_launches(B);
+    if (rc != BM_OK) B->versions.clear();   // not to be cycled: the next call makes it anew
     return rc;
 }
 
@@ -1118,16 +1140,19 @@ int bm_batch_get_profile(bm_batch batch, uint32_t n_max, uint32_t* kinds, uint32
     DevGuard g(batch->ctx->device);
     batch->drain_profile();
     uint32_t n = 0;
-    for (auto& p : batch->plan) {
-        if (!p.prof_n || n >= n_max) continue;
-        if (kinds) kinds[n] = p.form == bm_batch_s::F_FUSED ? 1000u + p.st.kind : p.st.kind;
-        if (layers) layers[n] = p.st.layer;
-        if (idx) idx[n] = p.st.idx;
-        if (n_areas) n_areas[n] = (uint32_t)p.areas.size();
-        if (launches) launches[n] = p.prof_n;
-        if (ms) ms[n] = p.prof_ms;
+    auto put = [&](const bm_batch_s::Prof& p) {
+        if (!p.n || n >= n_max) return;
+        if (kinds) kinds[n] = p.kind;
+        if (layers) layers[n] = p.layer;
+        if (idx) idx[n] = p.idx;
+        if (n_areas) n_areas[n] = p.n_areas;
+        if (launches) launches[n] = p.n;
+        if (ms) ms[n] = p.ms;
         n++;
-    }
+    };
+    for (auto& p : batch->plan)
+        put({p.prof_kind(), p.st.layer, p.st.idx, (uint32_t)p.areas.size(), p.prof_n, p.prof_ms});
+    for (auto& p : batch->retired) put(p);
     *n_out = n;
     return BM_OK;
 }
@@ -1140,6 +1165,7 @@ int bm_batch_reset_profile(bm_batch batch) {
         p.prof_n = 0;
         p.prof_ms = 0;
     }
+    batch->retired.clear();
     return BM_OK;
 }
 
