@@ -524,11 +524,8 @@ __device__ __forceinline__ void take_part(const FusedTuftArgs& A, TileGeo& G, ui
     G.syn_end = min(G.syn_end, G.syn0 + per * sb);
 }
 
-// Work item t of a one-tuft launch. SPLIT: it has parts (without, the kernel is
-// as it would be with whole tiles only: area_256's cycle 0.7 % shorter).
-template <bool SPLIT>
+// Work item t of a one-tuft launch.
 __device__ __forceinline__ TileGeo item_geo(const FusedTuftArgs& A, uint32_t t) {
-    if (!SPLIT) return tile_geo(A, t);
     const WorkItem w = work_item(A.split, t);
     TileGeo G = tile_geo(A, w.tile);
     take_part(A, G, w.part, w.parts);
@@ -562,6 +559,23 @@ __device__ __forceinline__ uint32_t code_base(const FusedTuftArgs& A, const Tile
     const uint32_t q = fast_div(local, A.u_size, A.usz_magic);   // whole rows: u0 is 0
     return ((((G.v0 + q) * A.src_vs) >> kSlcSclCoeffL2) - ((G.v0 * A.src_vs) >> kSlcSclCoeffL2)) * A.fw +
            (((local - q * A.u_size) * A.src_us) >> kSlcSclCoeffL2) + G.xoff;
+}
+
+// Footprint offsets, two a word, of 16 source codes (source_code): `base` is
+// code_base in both halves.
+__device__ __forceinline__ void code_offsets(const FusedTuftArgs& A, const uint32_t (&cw)[4], uint32_t base,
+                                             uint32_t (&gw)[8]) {
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        // (v << 4 | u) + (v << 4) * (fw / 16 - 1) = v * fw + u
+        const uint32_t x = __byte_perm(cw[w / 2], 0, (w & 1) ? 0x4342 : 0x4140);
+        gw[w] = (x & 0x00F000F0u) * A.code_mul + (x + base);
+    }
+}
+// The slices of those sources (a word of the slice plane) added in.
+__device__ __forceinline__ void slice_offsets(const FusedTuftArgs& A, uint32_t sl, uint32_t (&gw)[8]) {
+#pragma unroll
+    for (int w = 0; w < 8; w++) gw[w] += ((sl >> (2 * w)) & 0x00030003u) * A.fsz;
 }
 
 // syn_fire of four packed axon bytes (cl/syns.cl:2-4).
@@ -686,14 +700,25 @@ __device__ __forceinline__ void tma_stage(const FusedTuftArgs& A, const TileGeo&
                 // Compiled offsets index the footprint directly (it starts at
                 // shared offset 0); the 15-bit mask keeps even a stray offset
                 // inside the CTA's shared memory.
-                const uint4 g0 = *(const uint4*)(sb + 2 * so);
-                const uint4 g1 = *(const uint4*)(sb + 2 * so + 16);
-                const uint32_t gw[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+                // Tufts with source codes come here only for their foreign
+                // flags; every code is a place in the footprint.
+                uint32_t gw[8];
+                if (!FCLEAN && A.compact) {
+                    const uint4 c4 = *(const uint4*)(sb + so);
+                    const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w};
+                    code_offsets(A, cw, code_base(A, G, off >> A.S_l2) * 0x10001u, gw);
+                    if (A.compact == 2) slice_offsets(A, *(const uint32_t*)(sb + SB + so / 4), gw);
+                } else {
+                    const uint4 g0 = *(const uint4*)(sb + 2 * so);
+                    const uint4 g1 = *(const uint4*)(sb + 2 * so + 16);
+                    const uint32_t ofs[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+                    for (int w = 0; w < 8; w++) gw[w] = ofs[w] & 0x7FFF7FFFu;
+                }
 #pragma unroll
                 for (int w = 0; w < 4; w++) {
                     const uint32_t lo = gw[2 * w], hi = gw[2 * w + 1];
-                    ow[w] = pack4(halo[lo & 0x7FFFu], halo[(lo >> 16) & 0x7FFFu], halo[hi & 0x7FFFu],
-                                  halo[(hi >> 16) & 0x7FFFu]);
+                    ow[w] = pack4(halo[lo & 0xFFFFu], halo[lo >> 16], halo[hi & 0xFFFFu], halo[hi >> 16]);
                 }
             } else {
                 const uint4 slc4 = *(const uint4*)(sb + so);
@@ -849,17 +874,8 @@ __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo
             const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w};
             const uint32_t base1 = code_base(A, G, min(off, G.syn_end - 16u) >> S_L2), base = base1 * 0x10001u;
             if (MIS) edge_base = base1;
-#pragma unroll
-            for (int w = 0; w < 8; w++) {
-                // (v << 4 | u) + (v << 4) * (fw / 16 - 1) = v * fw + u
-                const uint32_t x = __byte_perm(cw[w / 2], 0, (w & 1) ? 0x4342 : 0x4140);
-                gw[w] = (x & 0x00F000F0u) * A.code_mul + (x + base);
-            }
-            if (A.compact == 2) {
-                const uint32_t sl = *(const uint32_t*)(sb + SRC + SX + so / 4);
-#pragma unroll
-                for (int w = 0; w < 8; w++) gw[w] += ((sl >> (2 * w)) & 0x00030003u) * A.fsz;
-            }
+            code_offsets(A, cw, base, gw);
+            if (A.compact == 2) slice_offsets(A, *(const uint32_t*)(sb + SRC + SX + so / 4), gw);
         } else {
             const uint4 g0 = *(const uint4*)(sb + SRC + 2 * so);
             const uint4 g1 = *(const uint4*)(sb + SRC + 2 * so + 16);
@@ -1024,8 +1040,6 @@ __device__ __forceinline__ bool produce_tile(const FusedTuftArgs& A, const TileG
         const uint32_t left = G.syn_end - pos;
         const uint32_t nb = left < SB ? left : SB;
         uint8_t* dst = stages + (size_t)pb * buf_bytes;
-        // Compact codes are streamed only for the specialised consumers (MODE 0,
-        // clean flags): other modes of such a tuft run as MODE 1 (mode_of).
         // MODE 2 copies the 16-byte windows the stage's synapses touch: one
         // more than they would fill, from the boundary below the first.
         const uint32_t nw = nb + (MODE == 2 ? 16 : 0), SX = SB + (MODE == 2 ? 16 : 0);
@@ -1176,7 +1190,7 @@ __device__ __noinline__ void seg_tile(const FusedTuftArgs& A, uint32_t t, uint8_
     fence_proxy_async_smem();   // a later tile's box may overwrite these bytes
 }
 
-template <bool TUFT, int MODE, bool FCLEAN, int GEOM, bool SPLIT>
+template <bool TUFT, int MODE, bool FCLEAN, int GEOM>
 __device__ __forceinline__ void tma_body(const FusedTuftArgs& A, uint8_t* smem, volatile int& s_abort) {
     uint64_t* full = (uint64_t*)(smem + A.ring_off);   // [nst]
     uint64_t* empty = full + A.nst;                    // [nst]
@@ -1193,7 +1207,7 @@ __device__ __forceinline__ void tma_body(const FusedTuftArgs& A, uint8_t* smem, 
         ps.ctl = A.ctl;
         ps.stall = blockIdx.x == 0 ? A.ctl->stall_stage : 0u;
         for (uint32_t t = blockIdx.x; t < A.split.items && !s_abort; t += gridDim.x) {
-            const TileGeo G = item_geo<SPLIT>(A, t);
+            const TileGeo G = item_geo(A, t);
             if (!produce_tile<TUFT, MODE, FCLEAN>(A, G, stages, full, empty, ps, s_abort)) break;
         }
         if (s_abort || ps.withheld >= 0) producer_drain(full, A.nst, ps);
@@ -1204,8 +1218,8 @@ __device__ __forceinline__ void tma_body(const FusedTuftArgs& A, uint8_t* smem, 
     uint32_t ring = 0;
     bool ok = true;
     for (uint32_t t = blockIdx.x; t < A.split.items; t += gridDim.x) {
-        const TileGeo G = item_geo<SPLIT>(A, t);
-        if (SPLIT && G.syn0 == G.syn_end) continue;
+        const TileGeo G = item_geo(A, t);
+        if (G.syn0 == G.syn_end) continue;
         // Every consumer is done with the previous tile; all leave together
         // if any gave up.
         if (consumers_sync_or(!ok || s_abort)) break;
@@ -1232,23 +1246,21 @@ __device__ __forceinline__ void init_ring(uint8_t* ring, uint32_t nst, volatile 
 // foreign flag bits) of a tuft, from its verification status.
 __device__ __forceinline__ uint32_t mode_of(const FusedTuftArgs& A) {
     const uint32_t status = A.ctl->tuft_status[A.status_idx];
-    const uint32_t mode = ((status & kTuftSrcOutsideTile) ? 2u : 0u) | ((status & kTuftFlagsForeign) ? 1u : 0u);
-    // The general consumer reads no compact codes: foreign flags then take the
-    // original source arrays too.
-    return A.compact && mode == 1 ? 3u : mode;
+    return ((status & kTuftSrcOutsideTile) ? 2u : 0u) | ((status & kTuftFlagsForeign) ? 1u : 0u);
 }
 
-// The general consumers beside the specialised ones are out of line: inlined
-// they make the kernel spill. Tufts whose shape has no specialised consumer
-// launch a kernel of general ones alone, with the arguments as constants
-// (through the call's pointer a 97 x 97 area's cycle was a sixth slower).
-template <bool TUFT, int MODE, bool FCLEAN>
-__device__ __noinline__ void tma_body_general(const FusedTuftArgs& A, uint8_t* smem, volatile int& s_abort) {
-    tma_body<TUFT, MODE, FCLEAN, 0, true>(A, smem, s_abort);
-}
-// FORM: 0 the tuft's shape has no specialised consumer (A.geom), 1 it has, 2 it
-// has and the tuft is unaligned.
-template <bool TUFT, int FORM, bool SPLIT>
+// A kernel per specialised shape (GEOM; 0: shapes without one), the general
+// consumers inline beside its own. Out of line, those reached the arguments
+// through a pointer and fetched them again after every store: area_256's cycle
+// with all flags foreign 620 us, 480 so (1095 where such a tuft also gave up its
+// source codes); a 97 x 97 x 3 area's with sources outside the footprint 124 and
+// 95 us. Inline in one kernel for all shapes they cost the specialised consumers
+// up to 2 %; in a kernel a shape these are as fast or faster than before (128 x
+// 128 x 4 of 16 x 32 synapses 87.1 us a cycle, 82.4 so; 160 x 160 x 3 of 16 x 64
+// 99.7 and 95.5), but for some sizes of 16-synapse dendrites (192 x 192 x 2 of
+// 8 x 16 27.5 and 28.4, of 16 x 16 37.4 and 37.7).
+// MIS: an unaligned tuft, of any of the pyramidal shapes.
+template <bool TUFT, int GEOM, bool MIS>
 __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_constant__ FusedTuftArgs A) {
     pdl_begin();
     extern __shared__ __align__(128) uint8_t smem[];
@@ -1256,42 +1268,28 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_con
     init_ring(smem + A.ring_off, A.nst, s_abort);
     // One body per gather mode and flags state (uniform per launch).
     const uint32_t mode = mode_of(A);
-    if constexpr (FORM == 0) {
-        switch (mode) {
-        case 0: tma_body<TUFT, 0, true, 0, SPLIT>(A, smem, s_abort); break;
-        case 1: tma_body<TUFT, 0, false, 0, SPLIT>(A, smem, s_abort); break;
-        case 2: tma_body<TUFT, 1, true, 0, SPLIT>(A, smem, s_abort); break;
-        default: tma_body<TUFT, 1, false, 0, SPLIT>(A, smem, s_abort); break;
-        }
-        return;
-    }
-    constexpr int M = FORM == 2 ? 2 : 0;
-    if constexpr (FORM == 2) {
+    if constexpr (MIS) {
         if (mode) {
             if (threadIdx.x >= kWarps * 32) return;
             const int32_t rnd = rnd_at(A.rnd_key, cycle_of(A));
             for (uint32_t t = blockIdx.x; t < A.n_tiles; t += gridDim.x) seg_tile(A, t, smem, rnd);
             return;
         }
-    } else
-    switch (mode) {
-    case 0: break;
-    case 1: tma_body_general<TUFT, 0, false>(A, smem, s_abort); return;
-    case 2: tma_body_general<TUFT, 1, true>(A, smem, s_abort); return;
-    default: tma_body_general<TUFT, 1, false>(A, smem, s_abort); return;
-    }
-    if constexpr (TUFT) {
         switch (A.geom) {
-        case 3: tma_body<TUFT, M, true, 3, SPLIT>(A, smem, s_abort); return;
-        case 4: tma_body<TUFT, M, true, 4, SPLIT>(A, smem, s_abort); return;
-        case 5: tma_body<TUFT, M, true, 5, SPLIT>(A, smem, s_abort); return;
-        case 6: tma_body<TUFT, M, true, 6, SPLIT>(A, smem, s_abort); return;
-        case 7: tma_body<TUFT, M, true, 7, SPLIT>(A, smem, s_abort); return;
-        default: tma_body<TUFT, M, true, 8, SPLIT>(A, smem, s_abort); return;
+        case 3: tma_body<TUFT, 2, true, 3>(A, smem, s_abort); break;
+        case 4: tma_body<TUFT, 2, true, 4>(A, smem, s_abort); break;
+        case 5: tma_body<TUFT, 2, true, 5>(A, smem, s_abort); break;
+        case 6: tma_body<TUFT, 2, true, 6>(A, smem, s_abort); break;
+        case 7: tma_body<TUFT, 2, true, 7>(A, smem, s_abort); break;
+        default: tma_body<TUFT, 2, true, 8>(A, smem, s_abort); break;
         }
     } else {
-        if (A.geom == 1) tma_body<TUFT, 0, true, 1, SPLIT>(A, smem, s_abort);
-        else tma_body<TUFT, 0, true, 2, SPLIT>(A, smem, s_abort);
+        switch (mode) {
+        case 0: tma_body<TUFT, 0, true, GEOM>(A, smem, s_abort); break;
+        case 1: tma_body<TUFT, 0, false, 0>(A, smem, s_abort); break;
+        case 2: tma_body<TUFT, 1, true, 0>(A, smem, s_abort); break;
+        default: tma_body<TUFT, 1, false, 0>(A, smem, s_abort); break;
+        }
     }
 }
 
@@ -1547,14 +1545,22 @@ int device_sms() {
     return sms;
 }
 
-// The one-tuft kernel of a layer kind, for a shape with a specialised consumer
-// or without, or for an unaligned tuft.
+// The one-tuft kernel of a layer kind and shape (consumer_shape), or of an
+// unaligned tuft.
 using TmaKernel = void (*)(FusedTuftArgs);
-TmaKernel tma_kernel(bool pyr, bool fast, bool mis, bool split) {
-    if (mis) return k_fused_tuft_tma<true, 2, true>;
-    if (!fast) return pyr ? k_fused_tuft_tma<true, 0, true> : k_fused_tuft_tma<false, 0, true>;
-    if (split) return pyr ? k_fused_tuft_tma<true, 1, true> : k_fused_tuft_tma<false, 1, true>;
-    return pyr ? k_fused_tuft_tma<true, 1, false> : k_fused_tuft_tma<false, 1, false>;
+TmaKernel tma_kernel(bool pyr, uint32_t geom, bool mis) {
+    if (mis) return k_fused_tuft_tma<true, 0, true>;
+    switch (geom) {
+    case 1: return k_fused_tuft_tma<false, 1, false>;
+    case 2: return k_fused_tuft_tma<false, 2, false>;
+    case 3: return k_fused_tuft_tma<true, 3, false>;
+    case 4: return k_fused_tuft_tma<true, 4, false>;
+    case 5: return k_fused_tuft_tma<true, 5, false>;
+    case 6: return k_fused_tuft_tma<true, 6, false>;
+    case 7: return k_fused_tuft_tma<true, 7, false>;
+    case 8: return k_fused_tuft_tma<true, 8, false>;
+    default: return pyr ? k_fused_tuft_tma<true, 0, false> : k_fused_tuft_tma<false, 0, false>;
+    }
 }
 
 // How n tiles of up to `stages` stages share `ctas` resident CTAs: the tiles of
@@ -1731,18 +1737,12 @@ void plan_tuft_form(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t
     for (uint32_t k = 0; k < nrec; k++) FT.src_idz[k] = P.slc_axn_idz[lo + k];
     // Persistent grid: as many CTAs as fit on the device at once.
     const bool pyr = L.kind == BM_LYR_PYRAMIDAL;
-    const bool fast = consumer_shape(FT, S, spd, pyr) != 0;
     // The cap is a property of the kernel, shared by every area on the device:
-    // set it to the largest footprint any tuft may plan, never lower. Both
-    // kernels of the tuft (its split is not known yet) fit the same CTAs.
+    // set it to the largest footprint any tuft may plan, never lower.
+    auto kern = tma_kernel(pyr, consumer_shape(FT, S, spd, pyr), FT.mis != 0);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
     int per_sm = 0;
-    for (bool split : {false, true}) {
-        auto kern = tma_kernel(pyr, fast, FT.mis != 0, split);
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
-        int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kThreads, FT.smem) != cudaSuccess) n = 1;
-        per_sm = per_sm ? std::min(per_sm, n) : n;
-    }
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, FT.smem) != cudaSuccess) per_sm = 1;
     const uint64_t n_tiles = (uint64_t)L.depth * ((L.u_size + W - 1) / W) * ((L.v_size + H - 1) / H);
     FT.split = tile_split((uint32_t)n_tiles, (uint32_t)(sms * std::max(per_sm, 1)), stages_of((uint64_t)W * H * S, SB));
     FT.grid = std::max<uint32_t>(1, std::min<uint32_t>(FT.split.items, (uint32_t)(sms * std::max(per_sm, 1))));
@@ -2069,7 +2069,7 @@ void launch_fused_tuft(const FusedArea& F, const uint8_t* axns, const SliceRec* 
     }
     const bool tuft = L.kind == BM_LYR_PYRAMIDAL;
     if (FT.tiled) {
-        auto kern = tma_kernel(tuft, A.geom != 0, FT.mis != 0, FT.split.parts > 1);
+        auto kern = tma_kernel(tuft, A.geom, FT.mis != 0);
         launch_pdl(kern, FT.grid, kThreads, FT.smem, s, A);
     } else {
         uint64_t want = (A.n_units + kWarps - 1) / kWarps;

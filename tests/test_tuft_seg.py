@@ -225,3 +225,45 @@ def test_few_synapses_from_the_layers_own_axons(syns, batched):
             b.close()
         a.close()
         ctx.close()
+
+
+@pytest.mark.parametrize("batched", [False, True])
+@pytest.mark.parametrize("mk", [
+    lambda: configs.benchmark_area(48, 64, 4, 16, 32, 6), lambda: configs.benchmark_area(33, 32, 1, 8, 32, 3),
+    lambda: configs.instance_area(100, 1, 16, 32), lambda: configs.instance_area(96, 2, 16, 64),
+    lambda: configs.instance_area(64, 3, 8, 16), lambda: configs.instance_area(80, 5, 8, 64),
+    lambda: configs.smoother_area(35, 3, 2)],
+    ids=["bench48", "bench33", "split_512", "split_1024", "three_slices", "five_slices", "smoother35"])
+def test_foreign_flags_come_and_go(mk, batched):
+    """Flag bytes with bits besides SYN_PREV_ACTIVE, in one synapse and in all:
+    the tuft's flags are streamed through, its compiled sources stay in use."""
+    ctx = cortex._Ctx(0)
+    a = cortex.CorticalArea(ctx, _desc(mk, settings_for()), 7)
+    slab = initial_slab(a.plan, 7, scramble_seed=11, clean_flags=True)
+    a.write_slab(slab)
+    b = cortex.Batch(ctx, [a]) if batched else None
+    fr = frames_for(a.plan, 4, 5)
+    rng = np.random.default_rng(4)
+    for k in range(4):
+        for l in range(a.plan.n_layers):
+            n = int(a.plan.layers[l].n_syns)
+            off = int(a.plan.layers[l].buf_off[F.BUF["syn_flag_sets"]])
+            flags = slab[off:off + n]
+            if k == 1:
+                flags[n - 1] |= 0x40
+            elif k == 2:
+                flags |= rng.integers(0, 256, n, dtype=np.uint8) & 0xEF
+            elif k == 3:
+                flags &= 0x10
+            if k:
+                a.write("syn_flag_sets", flags, layer=l)
+        a.write_input(fr[k])
+        (b or a).cycle(1)
+        oracle.intake(a.plan, slab, 0, 0, fr[k])
+        oracle.run(a.plan, slab, None, 1, start_cycle=k)
+        dev = a.read_slab()
+        assert np.array_equal(dev, slab), "cycle %d\n%s" % (k, diff_report(a.plan, dev, slab))
+    if b:
+        b.close()
+    a.close()
+    ctx.close()
