@@ -344,12 +344,15 @@ __device__ __forceinline__ TuftOut tuft_cell1_item(const uint8_t* __restrict__ a
     return {ts, (uint8_t)d_raw, braw, bid};
 }
 
-// A pyramidal tuft of a few synapses a cell, for cell c.
+// A tuft of a few synapses a cell, for cell c. (Spiny stellate layers, here with
+// two dendrites a cell or more, have no cell-tuft arrays and nothing to return.)
 __device__ __forceinline__ TuftOut tuft_cells_item(const uint8_t* __restrict__ axns,
                                                    const SliceRec* __restrict__ slices, const DevLayer& L, uint32_t t,
                                                    int32_t rnd, uint32_t c) {
-    if (L.tft[t].spt == 1) return tuft_cell1_item(axns, slices, L, t, rnd, c);
+    const bool pyr = L.kind == BM_LYR_PYRAMIDAL;
+    if (pyr && L.tft[t].spt == 1) return tuft_cell1_item(axns, slices, L, t, rnd, c);
     tuft_cell_item(axns, slices, L, t, rnd, c);
+    if (!pyr) return {};
     const uint64_t ci = L.tft[t].cel_idz + c;
     return {L.buf[BM_BUF_TFT_STATES][ci], L.buf[BM_BUF_TFT_BEST_DEN_STATES_RAW][ci],
             L.buf[BM_BUF_TFT_PREV_BEST_DEN_STATES_RAW][ci], L.buf[BM_BUF_TFT_PREV_BEST_DEN_IDS][ci]};

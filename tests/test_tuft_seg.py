@@ -267,3 +267,36 @@ def test_foreign_flags_come_and_go(mk, batched):
         b.close()
     a.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("batched", [False, True])
+@pytest.mark.parametrize("dens,syns", [(1, 1), (1, 4), (2, 1), (2, 2), (4, 1), (2, 4)])
+def test_spiny_stellate_cells_of_a_few_synapses(dens, syns, batched):
+    """Spiny stellate cells have no cell-tuft arrays: one dendrite a cell (with
+    the folded soma step) and several."""
+    src = M.TuftSourceLayer.define("iv").syn_reach(2).prevalence(1)
+    l2, a2 = _small(21, 2, M.CellScheme.pyramidal().tft(
+        M.TuftScheme.basal().proximal().dens_per_tft(2).syns_per_den(2).src_lyr(src)))
+    for layer in l2["visual"].layers:
+        if layer.name == "iv":
+            layer.cellular(M.CellScheme.spiny_stellate().tft(
+                M.TuftScheme.basal().proximal().dens_per_tft(dens).syns_per_den(syns)
+                .src_lyr(M.TuftSourceLayer.define("aff_in").syn_reach(3).prevalence(1))))
+    ctx = cortex._Ctx(0)
+    a = cortex.CorticalArea(ctx, M.area_desc("v1", l2, a2, settings_for()), 7)
+    assert int(a.plan.layers[0].tufts[0].syns_per_tft) == dens * syns
+    slab = initial_slab(a.plan, 7, scramble_seed=11, clean_flags=True)
+    a.write_slab(slab)
+    b = cortex.Batch(ctx, [a]) if batched else None
+    fr = frames_for(a.plan, 3, 5, active=0.2)
+    for k in range(3):
+        a.write_input(fr[k])
+        (b or a).cycle(1)
+        oracle.intake(a.plan, slab, 0, 0, fr[k])
+        oracle.run(a.plan, slab, None, 1, start_cycle=k)
+        dev = a.read_slab()
+        assert np.array_equal(dev, slab), "cycle %d\n%s" % (k, diff_report(a.plan, dev, slab))
+    if b:
+        b.close()
+    a.close()
+    ctx.close()
