@@ -1146,13 +1146,13 @@ int write_host_frame(bm_area_s* A, uint32_t input, const uint8_t* frame, size_t 
         size_t cap = 0;
         for (uint32_t i = 0; i < A->plan.n_inputs; i++) cap = std::max<size_t>(cap, A->plan.inputs[i].len);
         for (uint32_t k = 0; k < kUpSlots && e == cudaSuccess; k++) {
-            const size_t n = k < 2 ? cap : std::min(cap, kDirectBytes);
+            const size_t n = k < 2 ? cap : std::min(cap, kDirectFrame);
             e = cudaHostAlloc((void**)&A->up_host[k], std::max<size_t>(n, 1), cudaHostAllocMapped | cudaHostAllocPortable);
             if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&A->up_map[k], A->up_host[k], 0);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&A->up_taken[k], cudaEventDisableTiming);
         }
         for (int k = 0; k < 2 && e == cudaSuccess; k++) {
-            if (cap > kDirectBytes) e = cudaMalloc(&A->up_dev[k], cap);
+            if (cap > kDirectFrame) e = cudaMalloc(&A->up_dev[k], cap);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&A->up_loaded[k], cudaEventDisableTiming);
         }
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&A->up, cudaStreamNonBlocking);
@@ -1166,7 +1166,7 @@ int write_host_frame(bm_area_s* A, uint32_t input, const uint8_t* frame, size_t 
     if (len > A->up_cap) return set_err(BM_ERR_INVALID, "frame of %zu bytes exceeds the upload slot", len);
     std::vector<FramePiece> pieces;
     frame_pieces(A, input, 0, A->plan.inputs[input].len, pieces);
-    if (len <= kDirectBytes && pieces.size() <= kMaxCopyPieces) {
+    if (len <= kDirectFrame && pieces.size() <= kMaxCopyPieces) {
         const uint32_t k = A->up_next;
         A->up_next = (k + 1) % kUpSlots;
         // The intake of the slot's previous frame has run.
@@ -1535,7 +1535,7 @@ int bm_area_read_output(bm_area area, uint32_t output_idx, uint8_t* dst, size_t 
     cudaPointerAttributes at{};
     const bool pageable = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    if (pageable && len && len <= kDirectBytes) return read_back(area, src, dst, len);
+    if (pageable && len && len <= kDirectOutput) return read_back(area, src, dst, len);
     CU(cudaMemcpyAsync(dst, src, len, cudaMemcpyDeviceToHost, area->stream()));
     CU(cudaStreamSynchronize(area->stream()));
     return BM_OK;

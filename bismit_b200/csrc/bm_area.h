@@ -155,9 +155,20 @@ void ctx_release(bm_ctx c);   // frees the context with its last reference
 
 namespace bm {
 constexpr uint32_t kUpSlots = 4;
-// Frames and outputs of up to this many bytes cross the host link inside the
-// copy kernel of the cycling stream: no copy engine, no event between streams.
-constexpr size_t kDirectBytes = 256 << 10;
+// Frames of up to kDirectFrame bytes and outputs of up to kDirectOutput cross
+// the host link inside the copy kernel of the cycling stream: no copy engine, no
+// event between streams. In a loop of frame in, cycle, output back, us a cycle:
+//  * frames read in place / uploaded: 131,044 bytes into 362 x 362 x 4 551 / 435,
+//    250,000 into 500 x 500 x 4 983 / 786, 78,400 into 280 x 280 x 4 356 / 285,
+//    73,984 into 272 x 272 x 4 274 / 251; 90,601 into 301 x 301 x 2 194 / 195,
+//    262,144 into 512 x 512 x 1 218 / 222. (Which of the cycle's streams gets the
+//    SMs first turns on when the intake ends, and the uploaded frame's ends
+//    later.) Up to 64 KB the two are within 1 % of one another from 200 x 200 x 4
+//    on; a 64 x 64 area's loop is 13 us shorter with frame and output in place.
+//  * outputs written in place / downloaded: 160,000 bytes 164 / 170, 252,004 255
+//    / 264, 262,144 234 / 242.
+constexpr size_t kDirectFrame = 64 << 10;
+constexpr size_t kDirectOutput = 256 << 10;
 }  // namespace bm
 
 struct bm_area_s {
@@ -223,7 +234,7 @@ struct bm_area_s {
     bool front_last = false;      // the latest enqueued cycle used the front stream
     std::vector<bm_sampler_s*> samplers;   // per-cycle readback channels (bm_sampler.cu)
     // Host frames (bm_area_write_input) are copied into a pinned slot during
-    // the call. Up to kDirectBytes the intake kernel reads the slot itself,
+    // the call. Up to kDirectFrame the intake kernel reads the slot itself,
     // mapped into the device's address space; a slot is reused once that
     // kernel has run (up_taken). Larger frames are uploaded from slots 0 and 1
     // on `up` into a device slot while earlier cycles run, and moved into place
@@ -236,7 +247,7 @@ struct bm_area_s {
     bool up_direct[bm::kUpSlots] = {};     // the slot's last frame was read in place
     uint32_t up_next = 0, up_next_dev = 0;
     size_t up_cap = 0;
-    // Outputs read back up to kDirectBytes: a kernel writes them here.
+    // Outputs read back up to kDirectOutput: a kernel writes them here.
     uint8_t* out_host = nullptr;
     uint8_t* out_map = nullptr;
     size_t out_cap = 0;

@@ -1,6 +1,6 @@
-"""Host frames and outputs on both sides of the size up to which a copy kernel
-moves them over the host link (256 KB), in turns and without a wait between
-them, against the oracle or the state slab (tolerance: exact)."""
+"""Host frames and outputs on both sides of the sizes up to which a copy kernel
+moves them over the host link (64 KB, 256 KB), in turns and without a wait
+between them, against the oracle or the state slab (tolerance: exact)."""
 import numpy as np
 import pytest
 
@@ -10,7 +10,7 @@ from helpers import diff_report, initial_slab, settings_for
 
 pytestmark = pytest.mark.gpu
 
-LIMIT = 256 << 10
+LIMIT = 64 << 10
 
 
 def _two_inputs(src_side=252, src_depth=5, side=40):
@@ -47,9 +47,10 @@ def _two_inputs(src_side=252, src_depth=5, side=40):
 ORDERS = [(0, 1), (1, 0, 1, 1, 0), (0, 0, 1), (1, 1, 1, 1, 1, 0, 0, 0, 1), (0, 0, 0, 0, 1)]
 
 
-def test_large_and_small_frames_in_turns():
+@pytest.mark.parametrize("src_depth", [2, 5])
+def test_large_and_small_frames_in_turns(src_depth):
     ctx = cortex._Ctx(0)
-    lmaps, areas = _two_inputs()
+    lmaps, areas = _two_inputs(src_depth=src_depth)
     a = cortex.CorticalArea(ctx, M.area_desc("v1", lmaps, areas, settings_for()), 7)
     lens = [a.input_len(i) for i in range(2)]
     assert lens[0] > LIMIT > lens[1]
