@@ -524,8 +524,10 @@ __device__ __forceinline__ void take_part(const FusedTuftArgs& A, TileGeo& G, ui
     G.syn_end = min(G.syn_end, G.syn0 + per * sb);
 }
 
-// Work item t of a one-tuft launch.
+// Work item t of a one-tuft launch. SPLIT: it has parts.
+template <bool SPLIT>
 __device__ __forceinline__ TileGeo item_geo(const FusedTuftArgs& A, uint32_t t) {
+    if (!SPLIT) return tile_geo(A, t);
     const WorkItem w = work_item(A.split, t);
     TileGeo G = tile_geo(A, w.tile);
     take_part(A, G, w.part, w.parts);
@@ -1190,7 +1192,7 @@ __device__ __noinline__ void seg_tile(const FusedTuftArgs& A, uint32_t t, uint8_
     fence_proxy_async_smem();   // a later tile's box may overwrite these bytes
 }
 
-template <bool TUFT, int MODE, bool FCLEAN, int GEOM>
+template <bool TUFT, int MODE, bool FCLEAN, int GEOM, bool SPLIT>
 __device__ __forceinline__ void tma_body(const FusedTuftArgs& A, uint8_t* smem, volatile int& s_abort) {
     uint64_t* full = (uint64_t*)(smem + A.ring_off);   // [nst]
     uint64_t* empty = full + A.nst;                    // [nst]
@@ -1207,7 +1209,7 @@ __device__ __forceinline__ void tma_body(const FusedTuftArgs& A, uint8_t* smem, 
         ps.ctl = A.ctl;
         ps.stall = blockIdx.x == 0 ? A.ctl->stall_stage : 0u;
         for (uint32_t t = blockIdx.x; t < A.split.items && !s_abort; t += gridDim.x) {
-            const TileGeo G = item_geo(A, t);
+            const TileGeo G = item_geo<SPLIT>(A, t);
             if (!produce_tile<TUFT, MODE, FCLEAN>(A, G, stages, full, empty, ps, s_abort)) break;
         }
         if (s_abort || ps.withheld >= 0) producer_drain(full, A.nst, ps);
@@ -1218,8 +1220,8 @@ __device__ __forceinline__ void tma_body(const FusedTuftArgs& A, uint8_t* smem, 
     uint32_t ring = 0;
     bool ok = true;
     for (uint32_t t = blockIdx.x; t < A.split.items; t += gridDim.x) {
-        const TileGeo G = item_geo(A, t);
-        if (G.syn0 == G.syn_end) continue;
+        const TileGeo G = item_geo<SPLIT>(A, t);
+        if (SPLIT && G.syn0 == G.syn_end) continue;
         // Every consumer is done with the previous tile; all leave together
         // if any gave up.
         if (consumers_sync_or(!ok || s_abort)) break;
@@ -1256,11 +1258,14 @@ __device__ __forceinline__ uint32_t mode_of(const FusedTuftArgs& A) {
 // source codes); a 97 x 97 x 3 area's with sources outside the footprint 124 and
 // 95 us. Inline in one kernel for all shapes they cost the specialised consumers
 // up to 2 %; in a kernel a shape these are as fast or faster than before (128 x
-// 128 x 4 of 16 x 32 synapses 87.1 us a cycle, 82.4 so; 160 x 160 x 3 of 16 x 64
-// 99.7 and 95.5), but for some sizes of 16-synapse dendrites (192 x 192 x 2 of
-// 8 x 16 27.5 and 28.4, of 16 x 16 37.4 and 37.7).
+// 128 x 4 of 16 x 32 synapses 86.8 us a cycle, 82.1 so; 96 x 96 x 2 of 16 x 64
+// 33.1 and 31.5), but for some large sizes of 16 x 16 (256 x 256 x 2 64.7 and
+// 65.2).
+// SPLIT: the last round's tiles are cut into parts. Launches of whole tiles
+// alone are spared the registers (area_256's 8 cycles 2011 us, 2017 with the one
+// kernel for both; 192 x 192 x 2 of 8 x 16 27.3 and 28.8 a cycle).
 // MIS: an unaligned tuft, of any of the pyramidal shapes.
-template <bool TUFT, int GEOM, bool MIS>
+template <bool TUFT, int GEOM, bool MIS, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_constant__ FusedTuftArgs A) {
     pdl_begin();
     extern __shared__ __align__(128) uint8_t smem[];
@@ -1276,19 +1281,19 @@ __global__ void __launch_bounds__(kThreads, 3) k_fused_tuft_tma(const __grid_con
             return;
         }
         switch (A.geom) {
-        case 3: tma_body<TUFT, 2, true, 3>(A, smem, s_abort); break;
-        case 4: tma_body<TUFT, 2, true, 4>(A, smem, s_abort); break;
-        case 5: tma_body<TUFT, 2, true, 5>(A, smem, s_abort); break;
-        case 6: tma_body<TUFT, 2, true, 6>(A, smem, s_abort); break;
-        case 7: tma_body<TUFT, 2, true, 7>(A, smem, s_abort); break;
-        default: tma_body<TUFT, 2, true, 8>(A, smem, s_abort); break;
+        case 3: tma_body<TUFT, 2, true, 3, SPLIT>(A, smem, s_abort); break;
+        case 4: tma_body<TUFT, 2, true, 4, SPLIT>(A, smem, s_abort); break;
+        case 5: tma_body<TUFT, 2, true, 5, SPLIT>(A, smem, s_abort); break;
+        case 6: tma_body<TUFT, 2, true, 6, SPLIT>(A, smem, s_abort); break;
+        case 7: tma_body<TUFT, 2, true, 7, SPLIT>(A, smem, s_abort); break;
+        default: tma_body<TUFT, 2, true, 8, SPLIT>(A, smem, s_abort); break;
         }
     } else {
         switch (mode) {
-        case 0: tma_body<TUFT, 0, true, GEOM>(A, smem, s_abort); break;
-        case 1: tma_body<TUFT, 0, false, 0>(A, smem, s_abort); break;
-        case 2: tma_body<TUFT, 1, true, 0>(A, smem, s_abort); break;
-        default: tma_body<TUFT, 1, false, 0>(A, smem, s_abort); break;
+        case 0: tma_body<TUFT, 0, true, GEOM, SPLIT>(A, smem, s_abort); break;
+        case 1: tma_body<TUFT, 0, false, 0, SPLIT>(A, smem, s_abort); break;
+        case 2: tma_body<TUFT, 1, true, 0, SPLIT>(A, smem, s_abort); break;
+        default: tma_body<TUFT, 1, false, 0, SPLIT>(A, smem, s_abort); break;
         }
     }
 }
@@ -1546,21 +1551,25 @@ int device_sms() {
 }
 
 // The one-tuft kernel of a layer kind and shape (consumer_shape), or of an
-// unaligned tuft.
+// unaligned tuft. The specialised shapes have one for launches without parts.
 using TmaKernel = void (*)(FusedTuftArgs);
-TmaKernel tma_kernel(bool pyr, uint32_t geom, bool mis) {
-    if (mis) return k_fused_tuft_tma<true, 0, true>;
+template <bool SPLIT>
+TmaKernel shape_kernel(uint32_t geom) {
     switch (geom) {
-    case 1: return k_fused_tuft_tma<false, 1, false>;
-    case 2: return k_fused_tuft_tma<false, 2, false>;
-    case 3: return k_fused_tuft_tma<true, 3, false>;
-    case 4: return k_fused_tuft_tma<true, 4, false>;
-    case 5: return k_fused_tuft_tma<true, 5, false>;
-    case 6: return k_fused_tuft_tma<true, 6, false>;
-    case 7: return k_fused_tuft_tma<true, 7, false>;
-    case 8: return k_fused_tuft_tma<true, 8, false>;
-    default: return pyr ? k_fused_tuft_tma<true, 0, false> : k_fused_tuft_tma<false, 0, false>;
+    case 1: return k_fused_tuft_tma<false, 1, false, SPLIT>;
+    case 2: return k_fused_tuft_tma<false, 2, false, SPLIT>;
+    case 3: return k_fused_tuft_tma<true, 3, false, SPLIT>;
+    case 4: return k_fused_tuft_tma<true, 4, false, SPLIT>;
+    case 5: return k_fused_tuft_tma<true, 5, false, SPLIT>;
+    case 6: return k_fused_tuft_tma<true, 6, false, SPLIT>;
+    case 7: return k_fused_tuft_tma<true, 7, false, SPLIT>;
+    default: return k_fused_tuft_tma<true, 8, false, SPLIT>;
     }
+}
+TmaKernel tma_kernel(bool pyr, uint32_t geom, bool mis, bool split) {
+    if (mis) return k_fused_tuft_tma<true, 0, true, true>;
+    if (geom) return split ? shape_kernel<true>(geom) : shape_kernel<false>(geom);
+    return pyr ? k_fused_tuft_tma<true, 0, false, true> : k_fused_tuft_tma<false, 0, false, true>;
 }
 
 // How n tiles of up to `stages` stages share `ctas` resident CTAs: the tiles of
@@ -1738,9 +1747,14 @@ void plan_tuft_form(FusedTuft& FT, const bm_area_plan& P, uint32_t i, uint32_t t
     // Persistent grid: as many CTAs as fit on the device at once.
     const bool pyr = L.kind == BM_LYR_PYRAMIDAL;
     // The cap is a property of the kernel, shared by every area on the device:
-    // set it to the largest footprint any tuft may plan, never lower.
-    auto kern = tma_kernel(pyr, consumer_shape(FT, S, spd, pyr), FT.mis != 0);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+    // set it to the largest footprint any tuft may plan, never lower. Both
+    // kernels of the tuft (its split is not known yet) are held to the same
+    // registers, so the one with parts gives the CTAs of either.
+    TmaKernel kern = nullptr;
+    for (bool split : {false, true}) {
+        kern = tma_kernel(pyr, consumer_shape(FT, S, spd, pyr), FT.mis != 0, split);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+    }
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, FT.smem) != cudaSuccess) per_sm = 1;
     const uint64_t n_tiles = (uint64_t)L.depth * ((L.u_size + W - 1) / W) * ((L.v_size + H - 1) / H);
@@ -2069,7 +2083,7 @@ void launch_fused_tuft(const FusedArea& F, const uint8_t* axns, const SliceRec* 
     }
     const bool tuft = L.kind == BM_LYR_PYRAMIDAL;
     if (FT.tiled) {
-        auto kern = tma_kernel(tuft, A.geom, FT.mis != 0);
+        auto kern = tma_kernel(tuft, A.geom, FT.mis != 0, FT.split.parts > 1);
         launch_pdl(kern, FT.grid, kThreads, FT.smem, s, A);
     } else {
         uint64_t want = (A.n_units + kWarps - 1) / kWarps;
