@@ -17,8 +17,10 @@ BUILD = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libbismit_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+# Device code stays uncompressed: nvcc compresses an object past a size that the
+# tuft kernels reach, and unpacking it made a process's first area 10 ms later.
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
-         "--expt-relaxed-constexpr", "-Xptxas", "-warn-spills"]
+         "--expt-relaxed-constexpr", "-Xptxas", "-warn-spills", "--no-compress"]
 SOURCES = ["bm_api.cu", "bm_plain.cu", "bm_fused.cu", "bm_grow.cu", "bm_static.cu", "bm_batch.cu", "bm_server.cu", "bm_sampler.cu", "bm_encode.cu", "bm_layout.cpp"]
 
 
